@@ -284,29 +284,26 @@ int launch_decode(GemmParams p, const DeviceInfo& dev, const int32_t* packed, co
                            kDecStageK / 32, CU_TENSOR_MAP_SWIZZLE_NONE))
     return rc;
   const size_t smem = kDecWorkers * static_cast<size_t>(stages) * stage_bytes + fixed;
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, GemmParams);
+  static const Kernel kernels[3] = {w4a16_decode_kernel<16, false>, w4a16_decode_kernel<16, true>,
+                                    w4a16_decode_kernel<32, false>};
   static std::once_flag flags[64];
   static cudaError_t attr_result[64];
   int device = 0;
   CHORD_CUDA(cudaGetDevice(&device));
   std::call_once(flags[device & 63], [&] {
-    attr_result[device & 63] = cudaFuncSetAttribute(
-        w4a16_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin);
-    if (attr_result[device & 63] == cudaSuccess) {
-      attr_result[device & 63] = cudaFuncSetAttribute(
-          w4a16_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.max_smem_optin);
+    for (const Kernel kernel : kernels) {
+      const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  dev.max_smem_optin);
+      if (attr_result[device & 63] == cudaSuccess) attr_result[device & 63] = rc;
     }
   });
   if (attr_result[device & 63] != cudaSuccess) {
     return fail(kCudaError, "cudaFuncSetAttribute failed: %s",
                 cudaGetErrorString(attr_result[device & 63]));
   }
-  if (p.fuse_silu) {
-    CHORD_CUDA(launch_kernel(w4a16_decode_kernel<true>, dim3(grid), dim3(kDecThreads), smem, stream,
-                             p.pdl != 0, tm_w, tm_s, p));
-  } else {
-    CHORD_CUDA(launch_kernel(w4a16_decode_kernel<false>, dim3(grid), dim3(kDecThreads), smem, stream,
-                             p.pdl != 0, tm_w, tm_s, p));
-  }
+  const Kernel kernel = kernels[p.mma_n > 16 ? 2 : (p.fuse_silu ? 1 : 0)];
+  CHORD_CUDA(launch_kernel(kernel, dim3(grid), dim3(kDecThreads), smem, stream, p.pdl != 0, tm_w, tm_s, p));
   return kOk;
 }
 

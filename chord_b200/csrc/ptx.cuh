@@ -266,6 +266,25 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   return v;
 }
 
+// Four 8x8 BF16 matrices; lane l supplies the address of row l % 8 of matrix l / 8 and
+// receives, of matrix i, elements 2(l%4), 2(l%4)+1 of row l/4 in r[i].
+template <int kOffset>
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4+%5];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr), "n"(kOffset)
+               : "memory");
+}
+
+// D[16 rows, 8 columns] += A[16, 16] * B[16, 8]: BF16 operands, FP32 accumulation, all in
+// the warp's registers.
+__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // ------------------------------------------------------------ cp.async (LSU) --
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
@@ -429,52 +448,6 @@ __device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_
       : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
         "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
         "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
-// The 16x128b.x8 store with the final multiplication folded in: register 4j+{0,2} of the
-// operand is d[4j+{0,2}] times the low BF16 of the scale word and 4j+{1,3} times its high
-// BF16 (scale word s0 for j < 2, s1 for j >= 2).  Products and store live in one asm
-// statement so that the products are formed in the sixteen consecutive registers the
-// store reads, with no copies in between; the scale halves are broadcast with mov.b32
-// unpack/pack, which the assembler folds into the multiplies' operand selectors (a
-// byte-permute per broadcast, done outside, measured 2.5 % slower).
-__device__ __forceinline__ void tmem_st_16x128b_x8_scaled(uint32_t taddr, const uint32_t (&d)[16],
-                                                           uint32_t s0, uint32_t s1) {
-  asm volatile(
-      "{\n\t"
-      ".reg .b32 t<16>;\n\t"
-      ".reg .b16 a, b, c, e;\n\t"
-      ".reg .b32 s0l, s0h, s1l, s1h;\n\t"
-      "mov.b32 {a, b}, %17;\n\t"
-      "mov.b32 {c, e}, %18;\n\t"
-      "mov.b32 s0l, {a, a};\n\t"
-      "mov.b32 s0h, {b, b};\n\t"
-      "mov.b32 s1l, {c, c};\n\t"
-      "mov.b32 s1h, {e, e};\n\t"
-      "mul.rn.bf16x2 t0, %1, s0l;\n\t"
-      "mul.rn.bf16x2 t1, %2, s0h;\n\t"
-      "mul.rn.bf16x2 t2, %3, s0l;\n\t"
-      "mul.rn.bf16x2 t3, %4, s0h;\n\t"
-      "mul.rn.bf16x2 t4, %5, s0l;\n\t"
-      "mul.rn.bf16x2 t5, %6, s0h;\n\t"
-      "mul.rn.bf16x2 t6, %7, s0l;\n\t"
-      "mul.rn.bf16x2 t7, %8, s0h;\n\t"
-      "mul.rn.bf16x2 t8, %9, s1l;\n\t"
-      "mul.rn.bf16x2 t9, %10, s1h;\n\t"
-      "mul.rn.bf16x2 t10, %11, s1l;\n\t"
-      "mul.rn.bf16x2 t11, %12, s1h;\n\t"
-      "mul.rn.bf16x2 t12, %13, s1l;\n\t"
-      "mul.rn.bf16x2 t13, %14, s1h;\n\t"
-      "mul.rn.bf16x2 t14, %15, s1l;\n\t"
-      "mul.rn.bf16x2 t15, %16, s1h;\n\t"
-      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], "
-      "{t0, t1, t2, t3, t4, t5, t6, t7, t8, t9, t10, t11, t12, t13, t14, t15};\n\t"
-      "}\n"
-      :
-      : "r"(taddr), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]),
-        "r"(d[7]), "r"(d[8]), "r"(d[9]), "r"(d[10]), "r"(d[11]), "r"(d[12]), "r"(d[13]), "r"(d[14]),
-        "r"(d[15]), "r"(s0), "r"(s1)
       : "memory");
 }
 

@@ -368,21 +368,35 @@ __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t scale_lo, uint
   out[3] = bf16x2_mul(bf16x2_sub(v3, kBias), scale_hi);  // rows r+8, K-half 1
 }
 
-// First half of dequant_word: the four BF16 pairs (code - 8), exact, in the same order;
-// the multiplication by the scales is left to tmem_st_16x128b_x8_scaled.
-__device__ __forceinline__ void unbias_word(uint32_t w, uint32_t* out) {
-  constexpr uint32_t kMask = 0x000F000Fu;
-  constexpr uint32_t kMagic = 0x43004300u;
-  constexpr uint32_t kBias = 0x43084308u;
-  uint32_t v0, v1, v2, v3;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v0) : "r"(w), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v1) : "r"(w >> 4), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v2) : "r"(w >> 8), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v3) : "r"(w >> 12), "r"(kMask), "r"(kMagic));
-  out[0] = bf16x2_sub(v0, kBias);
-  out[2] = bf16x2_sub(v1, kBias);
-  out[1] = bf16x2_sub(v2, kBias);
-  out[3] = bf16x2_sub(v3, kBias);
+// dequant_word() with the two scales in one word (low half: rows r, high half: rows r+8).
+// They are broadcast with mov.b32 unpack/pack, which the assembler folds into the
+// multiplies' operand selectors (a byte-permute per broadcast measured 2.5 % slower).
+// out[] is the A fragment of mma.m16n8k16.
+__device__ __forceinline__ void dequant_fragment(uint32_t w, uint32_t scales, uint32_t (&out)[4]) {
+  asm("{\n\t"
+      ".reg .b32 v0, v1, v2, v3, s1, s2, s3, lo, hi;\n\t"
+      ".reg .b16 a, b;\n\t"
+      "mov.b32 {a, b}, %5;\n\t"
+      "mov.b32 lo, {a, a};\n\t"
+      "mov.b32 hi, {b, b};\n\t"
+      "shr.u32 s1, %4, 4;\n\t"
+      "shr.u32 s2, %4, 8;\n\t"
+      "shr.u32 s3, %4, 12;\n\t"
+      "lop3.b32 v0, %4, 0x000F000F, 0x43004300, 0xEA;\n\t"
+      "lop3.b32 v1, s1, 0x000F000F, 0x43004300, 0xEA;\n\t"
+      "lop3.b32 v2, s2, 0x000F000F, 0x43004300, 0xEA;\n\t"
+      "lop3.b32 v3, s3, 0x000F000F, 0x43004300, 0xEA;\n\t"
+      "sub.rn.bf16x2 v0, v0, %6;\n\t"
+      "sub.rn.bf16x2 v1, v1, %6;\n\t"
+      "sub.rn.bf16x2 v2, v2, %6;\n\t"
+      "sub.rn.bf16x2 v3, v3, %6;\n\t"
+      "mul.rn.bf16x2 %0, v0, lo;\n\t"
+      "mul.rn.bf16x2 %1, v2, hi;\n\t"
+      "mul.rn.bf16x2 %2, v1, lo;\n\t"
+      "mul.rn.bf16x2 %3, v3, hi;\n\t"
+      "}\n"
+      : "=&r"(out[0]), "=&r"(out[1]), "=&r"(out[2]), "=&r"(out[3])
+      : "r"(w), "r"(scales), "r"(0x43084308u));
 }
 
 // Ring position advanced without divisions (a lone issuing thread pays ~100
