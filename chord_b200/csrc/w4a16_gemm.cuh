@@ -972,201 +972,171 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   } else if (tiled_roles ? (warp == 1 || warp == 3) : (warp >= kFirstIssuerWarp && warp < kFirstDequantWarp)) {
     // ----------------------------------------------------------- MMA issuers --
     const uint32_t me = tiled_roles ? (warp >> 1) : warp - kFirstIssuerWarp;
-    if (me < ni && lane == 0 && rank == 0) {
+    // The whole warp walks the stages and waits; one elected lane issues.  A loop inside
+    // `if (lane == 0)` is divergent code to the compiler, which then moves every operand of
+    // every MMA (addresses, descriptors: all the same in all lanes) into the uniform registers
+    // the instruction reads, one by one, just before it: about 130 cycles per MMA.
+    // A wait that gives up is recorded in `bad` and tested once per stage; until then the
+    // issuer runs on, on whatever this CTA's operand buffers hold.
+    if (me < ni && rank == 0) {
       const uint64_t xdesc0 = ptx::smem_desc_k_sw128(ptx::smem_u32(smem_x));
       const uint64_t xdesc_stage = x_stage_bytes >> 4;  // descriptor address units are 16 bytes
       const uint64_t xdesc_half = x_half_bytes >> 4;
+      const uint32_t abort_addr = ptx::smem_u32(&sh.abort_flag);
+      const uint32_t xfull0 = ptx::smem_u32(&sh.xfull[0]), xempty0 = ptx::smem_u32(&sh.xempty[0]);
+      const uint32_t afull0 = ptx::smem_u32(&sh.afull[0]), aempty0 = ptx::smem_u32(&sh.aempty[0]);
       uint64_t xdesc = xdesc0;
       StageCursor cur, acur;
       XSubRing xring;
-      uint32_t it = 0, segc = 0;
-      bool ok = true;
-      while (ok && iter.next(seg)) {
+      uint32_t it = 0, segc = 0, bad = 0;
+      while (iter.next(seg)) {
         const TileInfo t = decode_tile(p, sh, seg.tile, rank);
         if (!t.valid) continue;
         const uint32_t d = d_bufs == 2 ? (segc & 1u) : 0u;
         const uint32_t dph = d_bufs == 2 ? ((segc >> 1) & 1u) : (segc & 1u);
-        if (!ptx::mbar_wait(ptx::smem_u32(&sh.dempty[d]), dph ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
+        ptx::mbar_wait_sticky(ptx::smem_u32(&sh.dempty[d]), dph ^ 1u, abort_addr, bad);
+        if (__any_sync(0xffffffffu, bad != 0)) break;
         ptx::tc_fence_after();
         const uint32_t d_addr = tmem_base + d_col0 + (d * ni + me) * d_cols;
-        const uint32_t idesc = ptx::idesc_bf16_f32(kBlockN << p.pair, static_cast<uint32_t>(t.mma_n));
+        // (through a shuffle: a value loaded from shared memory is not known to be uniform)
+        const uint32_t mma_n = __shfl_sync(0xffffffffu, static_cast<uint32_t>(t.mma_n), 0);
+        const uint32_t idesc = ptx::idesc_bf16_f32(kBlockN << p.pair, mma_n);
         uint32_t acc = 0;
-        const bool split = ksplit && t.mma_n <= 128;
+        const bool split = ksplit && mma_n <= 128;
         for (int32_t kb = seg.kb; kb < seg.ke; ++kb, ++it) {
-          if constexpr (kPair) {
-            // One MMA stream for both CTAs; every commit arrives on the barrier of each.
-            const uint32_t a = acur.s << 1;
-            const uint32_t aph = acur.ph;
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.xfull[cur.s]), cur.ph, abort_flag)) {
-              ok = false;
-              break;
+          const bool tail = k_tail_half && kb == k_iters - 1;  // no second K half
+          if (kPair || npair) {
+            // CTA pair: one MMA stream for both CTAs; every commit arrives on the barrier of
+            // each.  `npair`: the K block's two operand-ring entries belong to the tile's two
+            // weight blocks; this issuer takes the one of its block, with both K halves, into
+            // its accumulator.
+            uint32_t as = acur.s, aph = acur.ph;
+            if (!kPair) {
+              as += me;
+              if (as >= a_stages) {
+                as -= a_stages;
+                aph ^= 1u;
+              }
             }
-            const uint32_t a_addr = tmem_base + acur.s * kAColsPerStage;
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a]), aph, abort_flag)) {
-              ok = false;
-              break;
-            }
-            ptx::tc_fence_after();
-            ptx::mma_ts_k64_pair(d_addr, a_addr, xdesc, idesc, acc);
-            const uint32_t ae = ptx::smem_u32(&sh.aempty[a]);
-            ptx::mma_commit_pair(ae);
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a + 1]), aph, abort_flag)) {
-              ok = false;
-              break;
-            }
-            ptx::tc_fence_after();
-            if (!(k_tail_half && kb == k_iters - 1)) {
-              ptx::mma_ts_k64_pair(d_addr, a_addr + 32, xdesc + xdesc_half, idesc, 1);
-            }
-            acc = 1;
-            ptx::mma_commit_pair(ae + 8u);
-            ptx::mma_commit_pair(ptx::smem_u32(&sh.xempty[cur.s]));
-          } else if (npair) {
-            // The K block's two operand-ring entries belong to the tile's two weight blocks;
-            // this issuer takes the one of its block, with both K halves, into its accumulator.
-            uint32_t as = acur.s + me, aph = acur.ph;
-            if (as >= a_stages) {
-              as -= a_stages;
-              aph ^= 1u;
-            }
-            const uint32_t a = as << 1;
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.xfull[cur.s]), cur.ph, abort_flag)) {
-              ok = false;
-              break;
-            }
+            const uint32_t a_bar = as << 4;  // two 8-byte barriers per entry
             const uint32_t a_addr = tmem_base + as * kAColsPerStage;
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a]), aph, abort_flag)) {
-              ok = false;
-              break;
-            }
+            ptx::mbar_wait_sticky(xfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
+            ptx::mbar_wait_sticky(afull0 + a_bar, aph, abort_addr, bad);
             ptx::tc_fence_after();
-            ptx::mma_ts_k64(d_addr, a_addr, xdesc, idesc, acc);
-            ptx::mma_commit(ptx::smem_u32(&sh.aempty[a]));
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a + 1]), aph, abort_flag)) {
-              ok = false;
-              break;
+            if (ptx::elect_one()) {
+              if constexpr (kPair) {
+                ptx::mma_ts_k64_pair(d_addr, a_addr, xdesc, idesc, acc);
+                ptx::mma_commit_pair(aempty0 + a_bar);
+              } else {
+                ptx::mma_ts_k64(d_addr, a_addr, xdesc, idesc, acc);
+                ptx::mma_commit(aempty0 + a_bar);
+              }
             }
+            __syncwarp();
+            ptx::mbar_wait_sticky(afull0 + a_bar + 8u, aph, abort_addr, bad);
             ptx::tc_fence_after();
-            if (!(k_tail_half && kb == k_iters - 1)) {
-              ptx::mma_ts_k64(d_addr, a_addr + 32, xdesc + xdesc_half, idesc, 1);
+            if (ptx::elect_one()) {
+              if constexpr (kPair) {
+                if (!tail) ptx::mma_ts_k64_pair(d_addr, a_addr + 32, xdesc + xdesc_half, idesc, 1);
+                ptx::mma_commit_pair(aempty0 + a_bar + 8u);
+                ptx::mma_commit_pair(xempty0 + cur.s * 8u);
+              } else {
+                if (!tail) ptx::mma_ts_k64(d_addr, a_addr + 32, xdesc + xdesc_half, idesc, 1);
+                ptx::mma_commit(aempty0 + a_bar + 8u);
+                ptx::mma_commit(xempty0 + cur.s * 8u);
+              }
             }
+            __syncwarp();
             acc = 1;
-            ptx::mma_commit(ptx::smem_u32(&sh.aempty[a + 1]));
-            ptx::mma_commit(ptx::smem_u32(&sh.xempty[cur.s]));
-            acur.advance(a_stages);  // the other block's entry; the common advance below takes this one
+            if (!kPair) acur.advance(a_stages);  // the other block's entry; the common advance below takes this one
           } else if (ksplit) {
-            const uint32_t a = acur.s << 1;
+            const uint32_t a_bar = acur.s << 4;
             const uint32_t aph = acur.ph;
             uint32_t xslot = cur.s;       // barrier (and, with sub-slots, buffer) of this stage
             uint64_t xd = xdesc, xd_half = xdesc_half;
-            const bool two_slots = subslots && t.mma_n > 128;
+            const bool two_slots = subslots && mma_n > 128;
             if (subslots) {
               xslot = xring.take(two_slots, 2u * x_stages);
               xd = xdesc0 + xslot * (kSubBytes >> 4);
               xd_half = two_slots ? (kSubBytes >> 4) : (kSubBytes >> 5);
-              if (!ptx::mbar_wait(ptx::smem_u32(&sh.xfull[xslot]), xring.phase(xslot), abort_flag)) {
-                ok = false;
-                break;
-              }
+              ptx::mbar_wait_sticky(xfull0 + xslot * 8u, xring.phase(xslot), abort_addr, bad);
               xring.flip(xslot);
-            } else if (!ptx::mbar_wait(ptx::smem_u32(&sh.xfull[cur.s]), cur.ph, abort_flag)) {
-              ok = false;
-              break;
+            } else {
+              ptx::mbar_wait_sticky(xfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
             }
             if (p.x_load == kXLoadCpAsync) ptx::fence_proxy_async();
             const uint32_t a_addr = tmem_base + acur.s * kAColsPerStage;
-            const bool tail = k_tail_half && kb == k_iters - 1;
             if (me == 0) {
-              if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a]), aph, abort_flag)) {
-                ok = false;
-                break;
-              }
+              ptx::mbar_wait_sticky(afull0 + a_bar, aph, abort_addr, bad);
               ptx::tc_fence_after();
-              ptx::mma_ts(d_addr, a_addr, xd, idesc, acc);
-              ptx::mma_ts(d_addr, a_addr + 8, xd + 2, idesc, 1);
-              ptx::mma_ts(d_addr, a_addr + 16, xd + 4, idesc, 1);
-              ptx::mma_ts(d_addr, a_addr + 24, xd + 6, idesc, 1);
+              if (ptx::elect_one()) {
+                ptx::mma_ts_k64(d_addr, a_addr, xd, idesc, acc);
+                ptx::mma_commit(aempty0 + a_bar);
+              }
+              __syncwarp();
               acc = 1;
-              ptx::mma_commit(ptx::smem_u32(&sh.aempty[a]));
             }
             if (me == 0 ? !split : split) {
-              if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a + 1]), aph, abort_flag)) {
-                ok = false;
-                break;
-              }
+              ptx::mbar_wait_sticky(afull0 + a_bar + 8u, aph, abort_addr, bad);
               ptx::tc_fence_after();
-              if (!tail) {
-                const uint64_t xd1 = xd + xd_half;
-                ptx::mma_ts(d_addr, a_addr + 32, xd1, idesc, acc);
-                ptx::mma_ts(d_addr, a_addr + 40, xd1 + 2, idesc, 1);
-                ptx::mma_ts(d_addr, a_addr + 48, xd1 + 4, idesc, 1);
-                ptx::mma_ts(d_addr, a_addr + 56, xd1 + 6, idesc, 1);
-                acc = 1;
+              if (ptx::elect_one()) {
+                if (!tail) ptx::mma_ts_k64(d_addr, a_addr + 32, xd + xd_half, idesc, acc);
+                ptx::mma_commit(aempty0 + a_bar + 8u);
               }
-              ptx::mma_commit(ptx::smem_u32(&sh.aempty[a + 1]));
+              __syncwarp();
+              if (!tail) acc = 1;
             }
             // Both issuers account for the activation stage: a commit after MMAs of one's
             // own, a plain arrival otherwise.
-            if (me == 0 || split) ptx::mma_commit(ptx::smem_u32(&sh.xempty[xslot]));
-            else ptx::mbar_arrive(ptx::smem_u32(&sh.xempty[xslot]));
+            if (ptx::elect_one()) {
+              if (me == 0 || split) ptx::mma_commit(xempty0 + xslot * 8u);
+              else ptx::mbar_arrive(xempty0 + xslot * 8u);
+            }
+            __syncwarp();
           } else if ((it & (ni - 1)) == me) {
-            const uint32_t a = acur.s << 1;  // barrier of the first K half; the second is a + 1
+            const uint32_t a_bar = acur.s << 4;  // barrier of the first K half; the second follows it
             const uint32_t aph = acur.ph;
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.xfull[cur.s]), cur.ph, abort_flag)) {
-              ok = false;
-              break;
-            }
+            ptx::mbar_wait_sticky(xfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
             if (p.x_load == kXLoadCpAsync) ptx::fence_proxy_async();
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a]), aph, abort_flag)) {
-              ok = false;
-              break;
-            }
+            ptx::mbar_wait_sticky(afull0 + a_bar, aph, abort_addr, bad);
             ptx::tc_fence_after();
             const uint32_t a_addr = tmem_base + acur.s * kAColsPerStage;
-            ptx::mma_ts(d_addr, a_addr, xdesc, idesc, acc);
-            ptx::mma_ts(d_addr, a_addr + 8, xdesc + 2, idesc, 1);
-            ptx::mma_ts(d_addr, a_addr + 16, xdesc + 4, idesc, 1);
-            ptx::mma_ts(d_addr, a_addr + 24, xdesc + 6, idesc, 1);
-            ptx::mma_commit(ptx::smem_u32(&sh.aempty[a]));
-            if (!ptx::mbar_wait(ptx::smem_u32(&sh.afull[a + 1]), aph, abort_flag)) {
-              ok = false;
-              break;
+            if (ptx::elect_one()) {
+              ptx::mma_ts_k64(d_addr, a_addr, xdesc, idesc, acc);
+              ptx::mma_commit(aempty0 + a_bar);
             }
+            __syncwarp();
+            ptx::mbar_wait_sticky(afull0 + a_bar + 8u, aph, abort_addr, bad);
             ptx::tc_fence_after();
-            if (!(k_tail_half && kb == k_iters - 1)) {
-              const uint64_t xd1 = xdesc + xdesc_half;
-              ptx::mma_ts(d_addr, a_addr + 32, xd1, idesc, 1);
-              ptx::mma_ts(d_addr, a_addr + 40, xd1 + 2, idesc, 1);
-              ptx::mma_ts(d_addr, a_addr + 48, xd1 + 4, idesc, 1);
-              ptx::mma_ts(d_addr, a_addr + 56, xd1 + 6, idesc, 1);
+            if (ptx::elect_one()) {
+              if (!tail) ptx::mma_ts_k64(d_addr, a_addr + 32, xdesc + xdesc_half, idesc, 1);
+              ptx::mma_commit(aempty0 + a_bar + 8u);
+              ptx::mma_commit(xempty0 + cur.s * 8u);
             }
+            __syncwarp();
             acc = 1;
-            ptx::mma_commit(ptx::smem_u32(&sh.aempty[a + 1]));
-            ptx::mma_commit(ptx::smem_u32(&sh.xempty[cur.s]));
           }
           xdesc += xdesc_stage;
           cur.advance(x_stages);
           acur.advance(a_stages);
           if (cur.s == 0) xdesc = xdesc0;
+          if (__any_sync(0xffffffffu, bad != 0)) break;
         }
-        if (!ok) break;
+        if (__any_sync(0xffffffffu, bad != 0)) break;
         // One arrival per issuer and segment, also from an issuer that had no stage in it.
-        if constexpr (kPair) {
-          ptx::mma_commit_pair(ptx::smem_u32(&sh.dfull[d]));
-        } else if (acc != 0) {
-          ptx::mma_commit(ptx::smem_u32(&sh.dfull[d]));
-        } else {
-          ptx::mbar_arrive(ptx::smem_u32(&sh.dfull[d]));
+        if (ptx::elect_one()) {
+          if constexpr (kPair) {
+            ptx::mma_commit_pair(ptx::smem_u32(&sh.dfull[d]));
+          } else if (acc != 0) {
+            ptx::mma_commit(ptx::smem_u32(&sh.dfull[d]));
+          } else {
+            ptx::mbar_arrive(ptx::smem_u32(&sh.dfull[d]));
+          }
         }
+        __syncwarp();
         ++segc;
       }
-      if (!ok) {
-        sh.abort_flag = 1;
-        if (p.status) atomicOr(p.status, kStatusMmaTimeout);
-      }
+      if (__any_sync(0xffffffffu, bad != 0) && lane == 0 && p.status) atomicOr(p.status, kStatusMmaTimeout);
     }
     __syncwarp();
   } else if (warp >= kFirstDequantWarp && warp < kFirstEpilogueWarp) {
