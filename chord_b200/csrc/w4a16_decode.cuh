@@ -207,10 +207,10 @@ __device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, f
     }
     // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
     uint32_t a[4];
-    dequant_fragment(words[j].x, scales[j >> 1].x, a);
+    dequant_fragment(words[j].x, scales[j >> 1].x, a[0], a[1], a[2], a[3]);
 #pragma unroll
     for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
-    dequant_fragment(words[j].y, scales[j >> 1].y, a);
+    dequant_fragment(words[j].y, scales[j >> 1].y, a[0], a[1], a[2], a[3]);
 #pragma unroll
     for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
   }

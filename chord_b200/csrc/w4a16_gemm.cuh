@@ -335,44 +335,17 @@ __device__ __forceinline__ int32_t out_row_of(const GemmParams& p, const TileInf
   return (t.m0 + slot < t.limit) ? t.base + t.m0 + slot : -1;
 }
 
-__device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-
 // Expands one packed word (rows r and r+8, K offsets {2q, 2q+1, 2q+8, 2q+9} of a
 // K16 block; humming/kernel/repack.cuh:8-33) into four BF16 pairs
-// RN((code - 8) * scale), in tensor-memory store order:
-//   out[0] = (row r,   K 2q..2q+1)     out[1] = (row r+8, K 2q..2q+1)
-//   out[2] = (row r,   K 2q+8..2q+9)   out[3] = (row r+8, K 2q+8..2q+9)
-__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t scale_lo, uint32_t scale_hi,
-                                             uint32_t* out) {
-  constexpr uint32_t kMask = 0x000F000Fu;
-  constexpr uint32_t kMagic = 0x43004300u;   // BF16 128.0 in both halves
-  constexpr uint32_t kBias = 0x43084308u;    // BF16 136.0 in both halves
-  uint32_t v0, v1, v2, v3;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v0) : "r"(w), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v1) : "r"(w >> 4), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v2) : "r"(w >> 8), "r"(kMask), "r"(kMagic));
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v3) : "r"(w >> 12), "r"(kMask), "r"(kMagic));
-  out[0] = bf16x2_mul(bf16x2_sub(v0, kBias), scale_lo);  // rows r,   K-half 0
-  out[2] = bf16x2_mul(bf16x2_sub(v1, kBias), scale_lo);  // rows r,   K-half 1
-  out[1] = bf16x2_mul(bf16x2_sub(v2, kBias), scale_hi);  // rows r+8, K-half 0
-  out[3] = bf16x2_mul(bf16x2_sub(v3, kBias), scale_hi);  // rows r+8, K-half 1
-}
-
-// dequant_word() with the two scales in one word (low half: rows r, high half: rows r+8).
-// They are broadcast with mov.b32 unpack/pack, which the assembler folds into the
-// multiplies' operand selectors (a byte-permute per broadcast measured 2.5 % slower).
-// out[] is the A fragment of mma.m16n8k16.
-__device__ __forceinline__ void dequant_fragment(uint32_t w, uint32_t scales, uint32_t (&out)[4]) {
+// RN((code - 8) * scale), in the order of tcgen05.st.16x128b, which is also that of the A
+// fragment of mma.m16n8k16:
+//   d0 = (row r,   K 2q..2q+1)     d1 = (row r+8, K 2q..2q+1)
+//   d2 = (row r,   K 2q+8..2q+9)   d3 = (row r+8, K 2q+8..2q+9)
+// `scales`: low half for row r, high half for row r+8.  They are broadcast with mov.b32
+// unpack/pack, which the assembler folds into the multiplies' operand selectors (a
+// byte-permute per broadcast takes a slot of the half-rate integer pipe each).
+__device__ __forceinline__ void dequant_fragment(uint32_t w, uint32_t scales, uint32_t& d0, uint32_t& d1, uint32_t& d2,
+                                                 uint32_t& d3) {
   asm("{\n\t"
       ".reg .b32 v0, v1, v2, v3, s1, s2, s3, lo, hi;\n\t"
       ".reg .b16 a, b;\n\t"
@@ -395,7 +368,7 @@ __device__ __forceinline__ void dequant_fragment(uint32_t w, uint32_t scales, ui
       "mul.rn.bf16x2 %2, v1, lo;\n\t"
       "mul.rn.bf16x2 %3, v3, hi;\n\t"
       "}\n"
-      : "=&r"(out[0]), "=&r"(out[1]), "=&r"(out[2]), "=&r"(out[3])
+      : "=&r"(d0), "=&r"(d1), "=&r"(d2), "=&r"(d3)
       : "r"(w), "r"(scales), "r"(0x43084308u));
 }
 
@@ -1185,12 +1158,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       for (int j = 0; j < 4; ++j) {
         const uint2 sc = scales[j >> 1];
         // sc.x = {slab A row r, slab A row r+8}; sc.y = same for slab B.
-        const uint32_t a_lo = __byte_perm(sc.x, 0, 0x1010);
-        const uint32_t a_hi = __byte_perm(sc.x, 0, 0x3232);
-        const uint32_t b_lo = __byte_perm(sc.y, 0, 0x1010);
-        const uint32_t b_hi = __byte_perm(sc.y, 0, 0x3232);
-        dequant_word(words[j].x, a_lo, a_hi, lo + 4 * j);
-        dequant_word(words[j].y, b_lo, b_hi, hi + 4 * j);
+        dequant_fragment(words[j].x, sc.x, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+        dequant_fragment(words[j].y, sc.y, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
       }
     };
     // Waits for the slot to be free, then stores one K half: lo to TMEM lanes 0-15 of
