@@ -199,8 +199,10 @@ int launch_with_groups(const CUtensorMap& tm_w, const CUtensorMap& tm_s, const C
 }
 
 // `indexed` with routing blocks of 64 rows or more: the routed activation rows are first
-// copied into slot order (row s of the copy = the row sorted_ids[s] names, zeros for a
-// sentinel), so that the GEMM loads them as TMA boxes like `contiguous` does.  Two
+// copied into slot order (row s of the copy = the row sorted_ids[s] names; rows of sentinels
+// are left as they are: a token's column of the product depends on its own row alone, and
+// the columns of sentinels are not stored), so that the GEMM loads them as TMA boxes like
+// `contiguous` does.  Two
 // gathering warps cannot feed 64..256-row tiles: at 85 rows per tile they were the
 // bottleneck (2400 of 2600 cycles per stage), at 256 rows seven times slower than the
 // MMAs.  The copy costs one read and one write of the routed rows (HBM-bound, <2 % of
@@ -217,12 +219,10 @@ gather_routed_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __
     const int32_t id = __ldg(sorted_ids + slot);
     const int32_t row = (id >= 0 && id < out_rows) ? id / top_k : x_rows;
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(slot) * k);
-    if (row < x_rows) {
-      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * k);
-      for (int32_t i = lane; i < k / 8; i += 32) dst[i] = __ldg(src + i);
-    } else {
-      for (int32_t i = lane; i < k / 8; i += 32) dst[i] = make_uint4(0, 0, 0, 0);
-    }
+    if (row >= x_rows) continue;  // the rows of the copy that no id names are not stored by the GEMM
+    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * k);
+#pragma unroll 4
+    for (int32_t i = lane; i < k / 8; i += 32) dst[i] = __ldg(src + i);
   }
 }
 
