@@ -174,7 +174,8 @@ struct SegmentIterator {
   int64_t units, u0, u1;
   int32_t geff;
 
-  __host__ __device__ void init(int32_t tiles, int32_t k_iters, int32_t grid_, int32_t cta_) {
+  __host__ __device__ void init(int32_t tiles, int32_t k_iters, int32_t grid_, int32_t cta_,
+                                int32_t min_slice = 8) {
     grid = grid_;
     cta = cta_;
     ki = k_iters;
@@ -188,9 +189,9 @@ struct SegmentIterator {
     dp_tiles = dp_waves * grid;
     wave = 0;
     units = static_cast<int64_t>(sk_tiles) * ki;
-    // No slice shorter than eight k-blocks (unless the whole tail is): a finer split costs
-    // more in partial sums and per-slice set-up than the extra parallelism returns.
-    const int64_t slices = units / 8 > 0 ? units / 8 : (units > 0 ? 1 : 0);
+    // No slice shorter than `min_slice` k-blocks (unless the whole tail is): a finer split
+    // costs more in partial sums and per-slice set-up than the extra parallelism returns.
+    const int64_t slices = units / min_slice > 0 ? units / min_slice : (units > 0 ? 1 : 0);
     geff = slices < grid ? static_cast<int32_t>(slices) : grid;
     if (cta < geff) {
       u0 = cta * units / geff;
