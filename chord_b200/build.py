@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PACKAGE_DIR = Path(__file__).resolve().parent
@@ -30,7 +31,7 @@ def _nvcc() -> str:
 
 
 def _newest_source_mtime() -> float:
-    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
+    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(CSRC.glob("*.c"))
     files.append(PACKAGE_DIR.parent / "include" / "chord_b200.h")
     return max(f.stat().st_mtime for f in files if f.exists())
 
@@ -54,6 +55,23 @@ def _compile(nvcc: str, src: str, obj_dir: Path, verbose: bool) -> Path:
     return obj
 
 
+def _build_call_module(verbose: bool) -> None:
+    """The optional ``_call`` extension module (csrc/pycall.c); without Python's headers or a C
+    compiler the library is called through ctypes instead."""
+    headers = Path(sysconfig.get_paths()["include"])
+    gcc = shutil.which(os.environ.get("CC", "gcc"))
+    if gcc is None or not (headers / "Python.h").exists():
+        return
+    out = PACKAGE_DIR / ("_call" + sysconfig.get_config_var("EXT_SUFFIX"))
+    tmp = out.with_suffix(".tmp")
+    cmd = [gcc, "-O2", "-Wall", "-fPIC", "-shared", f"-I{headers}", str(CSRC / "pycall.c"), "-o", str(tmp)]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode == 0:
+        os.replace(tmp, out)
+    elif verbose:
+        sys.stderr.write(proc.stderr)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile the CUDA sources for sm_100a and link ``libchord_b200.so`` in-tree."""
     if not force and is_fresh():
@@ -63,6 +81,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     obj_dir.mkdir(exist_ok=True)
     with concurrent.futures.ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
         objs = list(pool.map(lambda s: _compile(nvcc, s, obj_dir, verbose), SOURCES))
+    _build_call_module(verbose)
     tmp = LIB_PATH.with_suffix(".so.tmp")
     cmd = [nvcc, *ARCH_FLAGS, "-shared", "-o", str(tmp), *map(str, objs)]
     proc = subprocess.run(cmd, capture_output=True, text=True)

@@ -44,8 +44,9 @@ constexpr int kDecMaxStages = 6;
 constexpr int kDecMaxTokens = 32;
 constexpr int kDecWorkers = 4;                        // workers per CTA
 constexpr int kDecThreads = 32 * (kDecWorkers + 4 * kDecWorkers);  // feeders, computing warps
-// Shortest stream-K slice in K blocks (a fused gate_up tile has two stages per K block).  8 experts of 1024 x 512, 64 tokens (four stages per
-// tile): 12.8 us with slices of eight stages, 8.7 us with four; longer K: no difference.
+// Shortest stream-K slice in K blocks (a fused gate_up tile has two stages per K block).
+// 8 experts of 1024 x 512, 64 tokens (four blocks per tile): 12.8 us with slices of eight,
+// 8.7 us with four; longer K: no difference.
 constexpr int kDecMinSlice = 4;
 constexpr int kDecPitch = 40;  // BF16 per token row of the epilogue buffer: 32 rows, padded against bank conflicts
 

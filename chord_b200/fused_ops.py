@@ -31,7 +31,7 @@ def silu_mul(gate_up: torch.Tensor, *, sorted_ids: torch.Tensor | None = None,
     elif (outputs.dtype != torch.bfloat16 or tuple(outputs.shape) != (rows, inter)
           or not outputs.is_contiguous() or outputs.device != device):
         raise ValueError(f"outputs must be contiguous BF16 {(rows, inter)} on {device}")
-    lib = _lib.load()
+    lib = _lib.native()
     with _lib.on_device(device):
         stream = _lib.stream_handle(device)
         if sorted_ids is None:
@@ -67,7 +67,7 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_m: int, num_experts: int,
     sorted_ids = torch.empty(blocks * block_m, dtype=torch.int32, device=device)
     expert_ids = torch.empty(blocks, dtype=torch.int32, device=device)
     num_tokens_padded = torch.empty(1, dtype=torch.int32, device=device)
-    lib = _lib.load()
+    lib = _lib.native()
     with _lib.on_device(device):
         _lib.check(lib.chord_b200_moe_align_block_size(
             topk_ids.data_ptr(), numel, expert_base, num_experts, block_m,

@@ -28,7 +28,7 @@ def _operands(inputs, weight):
 
 
 def masked_tile_m(expected_m: int) -> int:
-    return int(_lib.load().chord_b200_masked_tile_m(expected_m))
+    return int(_lib.native().chord_b200_masked_tile_m(expected_m))
 
 
 def w4a16_masked(
@@ -73,7 +73,7 @@ def w4a16_masked(
     else:
         _checks.bf16_output(outputs, (groups * max_m, weight.n), device, exact_shape=False)
     tile_m = masked_tile_m(expected_m)
-    lib = _lib.load()
+    lib = _lib.native()
     with _lib.on_device(device):
         locks, workspace, ws_bytes = gemm_scratch(device, tile_m, None)
         _lib.check(lib.chord_b200_masked(
@@ -114,7 +114,7 @@ def w4a16_contiguous(
         outputs = torch.empty((m, weight.n), dtype=torch.bfloat16, device=device)
     else:
         _checks.bf16_output(outputs, (m, weight.n), device, exact_shape=False)
-    lib = _lib.load()
+    lib = _lib.native()
     with _lib.on_device(device):
         locks, workspace, ws_bytes = gemm_scratch(device, 256, None)
         _lib.check(lib.chord_b200_contiguous(

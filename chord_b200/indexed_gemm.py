@@ -117,7 +117,7 @@ def select_block_m(shape_n: int, shape_k: int, num_experts: int, routed_m: int) 
     _checks.integer("shape_k", shape_k, minimum=1)
     _checks.integer("num_experts", num_experts, minimum=1)
     _checks.integer("routed_m", routed_m, minimum=0, type_error=True)
-    return int(_lib.load().chord_b200_indexed_block_m(shape_n, shape_k, num_experts, routed_m))
+    return int(_lib.native().chord_b200_indexed_block_m(shape_n, shape_k, num_experts, routed_m))
 
 
 def indexed_block_m(weight: PreparedWeight, num_tokens: int, top_k: int, *, device=None,
@@ -189,7 +189,7 @@ def w4a16_indexed(
         _checks.routing_contract(sorted_ids, expert_ids, num_tokens_padded, block_m, routed_m,
                                  num_experts)
 
-    lib = _lib.load()
+    lib = _lib.native()
     with _lib.on_device(device):
         locks, workspace, ws_bytes = gemm_scratch(device, block_m, locks, sorted_ids.numel(), shape_k)
         _lib.check(lib.chord_b200_indexed(
@@ -247,7 +247,7 @@ def indexed_gate_up_silu(
         outputs = torch.empty((routed_m, inter), dtype=torch.bfloat16, device=device)
     else:
         _checks.bf16_output(outputs, (routed_m, inter), device, exact_shape=True)
-    lib = _lib.load()
+    lib = _lib.native()
     if not lib.chord_b200_gate_up_silu_supported(shape_n, shape_k, block_m):
         gate_up = w4a16_indexed(activation, weight, sorted_ids, expert_ids, num_tokens_padded, top_k,
                                 locks=locks, block_m=block_m)
