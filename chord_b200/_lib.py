@@ -106,7 +106,7 @@ def native():
     """The entry points for calls with plain integer arguments (addresses included): through
     the ``_call`` extension module where it was built, otherwise the ctypes functions of
     :func:`load`.  ctypes spends 4.5 us on converting the 21 arguments of ``indexed``, the
-    module 0.5 us; a pass of four calls on a small layer goes from 71 to 47 us with this and
+    module less than 1 us; a pass of four calls on a small layer goes from 71 to 47 us with this and
     the cheaper stream look-up."""
     global _NATIVE
     if _NATIVE is None:

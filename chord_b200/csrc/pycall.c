@@ -1,6 +1,6 @@
 /* Calls a C-ABI entry point of the library from Python: call(address, arg, ...) with
  * integer arguments, returning its int result.  ctypes does the same at about 4.5 us for the
- * 21 arguments of `indexed` (an argument object each); this takes a tenth of that, on a path
+ * 21 arguments of `indexed` (an argument object each); this takes less than 1 us, on a path
  * that is called once per GEMM.  Every parameter of the entry points it serves is a pointer, an
  * int64_t or an int, which the x86-64 and AArch64 calling conventions pass alike in the
  * registers and eight-byte stack slots of an int64_t; arguments past the callee's last one are

@@ -1,5 +1,4 @@
-// Routing alignment (moe_align_block_size) as a device routine shared by the
-// stand-alone kernel and the expert-parallel receive step.
+// Routing alignment (moe_align_block_size) as a device routine.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -7,94 +6,122 @@
 
 namespace chord {
 
-constexpr int kAlignWarps = 16;
+constexpr int kAlignWarps = 32;
+constexpr int kAlignWarpsFew = 16;
 
 // Dynamic shared memory the routine needs for `num_experts` experts.
-inline size_t moe_align_smem_bytes(int64_t num_experts) {
-  return (static_cast<size_t>(kAlignWarps) * num_experts + num_experts + 1) * 4;
+inline size_t moe_align_smem_bytes(int64_t num_experts, int warps) {
+  return (static_cast<size_t>(warps) * num_experts + num_experts + 1) * 4;
 }
 
-// One CTA of kAlignWarps warps (CUDA form of the reference's align_routing_blocks,
+// One CTA of kWarps warps (CUDA form of the reference's align_routing_blocks,
 // tests/generators.py:192-230).  Pass 1 counts routes per (warp, expert); the per-expert
 // totals give the padded block layout; pass 2 replays the same walk and places every id
 // at expert offset + routes of lower warps + routes seen so far by this warp, so ids
 // inside an expert stay ascending and the result is deterministic.  `sentinel` pads the
-// blocks (any value >= the number of routed rows the GEMM is told about).  Entries are
-// read past L1, so ids another GPU wrote before a flag this CTA has acquired are seen.
+// blocks (any value >= the number of routed rows the GEMM is told about).
+//
+// Bound by latency: one CTA, every step waiting for L2 or shared memory.  A warp loads its ids
+// kBatch rounds of 32 ahead (one L2 round trip per batch instead of one per round) and keeps
+// them for pass 2 where it has no more than one batch; the offsets come from a warp scan.
+template <int kWarps, int kBatch>
 __device__ __forceinline__ void moe_align_block(const int32_t* topk_ids, int32_t numel, int32_t sentinel,
                                                 int32_t expert_base, int32_t num_experts,
                                                 int32_t block_m, int32_t* sorted_ids,
                                                 int32_t sorted_cap, int32_t* expert_ids,
                                                 int32_t expert_cap, int32_t* num_tokens_padded) {
   extern __shared__ int32_t align_smem[];
-  int32_t* counts = align_smem;                              // [kAlignWarps][num_experts]
-  int32_t* offsets = align_smem + kAlignWarps * num_experts;  // [num_experts + 1]
+  int32_t* counts = align_smem;                          // [kWarps][num_experts]
+  int32_t* offsets = align_smem + kWarps * num_experts;  // [num_experts + 1]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kAlignWarps * num_experts; i += blockDim.x) counts[i] = 0;
-  __syncthreads();
+  for (int i = threadIdx.x; i < kWarps * num_experts; i += blockDim.x) counts[i] = 0;
 
-  const int32_t per_warp = ((numel + kAlignWarps - 1) / kAlignWarps + 31) / 32 * 32;
+  // Local expert of the ids i + 32 u + lane, or -1.
+  const int32_t per_warp = ((numel + kWarps - 1) / kWarps + 31) / 32 * 32;
   const int32_t begin = warp * per_warp;
   const int32_t end = min(numel, begin + per_warp);
-  for (int32_t i = begin; i < end; i += 32) {
-    const int32_t idx = i + lane;
-    int32_t e = -1;
-    if (idx < end) {
-      e = __ldcg(topk_ids + idx) - expert_base;
-      if (e < 0 || e >= num_experts) e = -1;
+  int32_t e[kBatch];
+  auto load = [&](int32_t i) {
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int32_t idx = i + 32 * u + lane;
+      e[u] = idx < end ? __ldcg(topk_ids + idx) : -1;
     }
-    const uint32_t peers = __match_any_sync(0xffffffffu, e);
-    if (e >= 0 && lane == __ffs(peers) - 1) counts[warp * num_experts + e] += __popc(peers);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const uint32_t local = static_cast<uint32_t>(e[u]) - static_cast<uint32_t>(expert_base);
+      e[u] = (i + 32 * u + lane < end && local < static_cast<uint32_t>(num_experts)) ? static_cast<int32_t>(local) : -1;
+    }
+  };
+  constexpr int32_t kStep = 32 * kBatch;
+  int32_t* mine = counts + warp * num_experts;
+  if (begin < end) load(begin);
+  __syncthreads();
+  for (int32_t i = begin; i < end; i += kStep) {
+    if (i != begin) load(i);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (e[u] >= 0) atomicAdd(mine + e[u], 1);
+    }
   }
   __syncthreads();
 
   // Per expert: totals, and per-warp counts turned into exclusive prefixes.
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+  for (int x = threadIdx.x; x < num_experts; x += blockDim.x) {
     int32_t run = 0;
-    for (int w = 0; w < kAlignWarps; ++w) {
-      const int32_t c = counts[w * num_experts + e];
-      counts[w * num_experts + e] = run;
+#pragma unroll 8
+    for (int w = 0; w < kWarps; ++w) {
+      const int32_t c = counts[w * num_experts + x];
+      counts[w * num_experts + x] = run;
       run += c;
     }
-    offsets[e] = (run + block_m - 1) / block_m * block_m;
+    offsets[x] = (run + block_m - 1) / block_m * block_m;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == 0) {
     int32_t acc = 0;
-    for (int e = 0; e < num_experts; ++e) {
-      const int32_t padded = offsets[e];
-      offsets[e] = acc;
-      acc += padded;
+    for (int x0 = 0; x0 < num_experts; x0 += 32) {
+      const int32_t padded = x0 + lane < num_experts ? offsets[x0 + lane] : 0;
+      int32_t scan = padded;  // inclusive
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int32_t below = __shfl_up_sync(0xffffffffu, scan, d);
+        if (lane >= d) scan += below;
+      }
+      if (x0 + lane < num_experts) offsets[x0 + lane] = acc + scan - padded;
+      acc += __shfl_sync(0xffffffffu, scan, 31);
     }
-    offsets[num_experts] = acc;
-    *num_tokens_padded = acc < sorted_cap ? acc : sorted_cap / block_m * block_m;
+    if (lane == 0) {
+      offsets[num_experts] = acc;
+      *num_tokens_padded = acc < sorted_cap ? acc : sorted_cap / block_m * block_m;
+    }
   }
   __syncthreads();
   const int32_t total = min(offsets[num_experts], sorted_cap / block_m * block_m);
   for (int32_t i = threadIdx.x; i < total; i += blockDim.x) sorted_ids[i] = sentinel;
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-    for (int32_t b = offsets[e] / block_m; b < offsets[e + 1] / block_m; ++b) {
-      if (b < expert_cap) expert_ids[b] = e;
+  for (int x = threadIdx.x; x < num_experts; x += blockDim.x) {
+    for (int32_t b = offsets[x] / block_m; b < offsets[x + 1] / block_m; ++b) {
+      if (b < expert_cap) expert_ids[b] = x;
     }
   }
   __syncthreads();
 
-  for (int32_t i = begin; i < end; i += 32) {
-    const int32_t idx = i + lane;
-    int32_t e = -1;
-    if (idx < end) {
-      e = __ldcg(topk_ids + idx) - expert_base;
-      if (e < 0 || e >= num_experts) e = -1;
+  for (int32_t i = begin; i < end; i += kStep) {
+    // (the ids of a single batch are still in the registers)
+    if (end - begin > kStep) load(i);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (i + 32 * u >= end) break;
+      const uint32_t peers = __match_any_sync(0xffffffffu, e[u]);
+      if (e[u] >= 0) {
+        const int32_t rank = __popc(peers & ((1u << lane) - 1u));
+        const int32_t pos = offsets[e[u]] + mine[e[u]] + rank;
+        if (pos < total) sorted_ids[pos] = i + 32 * u + lane;
+      }
+      __syncwarp();
+      if (e[u] >= 0 && lane == __ffs(peers) - 1) mine[e[u]] += __popc(peers);
+      __syncwarp();
     }
-    const uint32_t peers = __match_any_sync(0xffffffffu, e);
-    if (e >= 0) {
-      const int32_t rank = __popc(peers & ((1u << lane) - 1u));
-      const int32_t pos = offsets[e] + counts[warp * num_experts + e] + rank;
-      if (pos < total) sorted_ids[pos] = idx;
-    }
-    __syncwarp();
-    if (e >= 0 && lane == __ffs(peers) - 1) counts[warp * num_experts + e] += __popc(peers);
-    __syncwarp();
   }
 }
 
