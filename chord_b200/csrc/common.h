@@ -71,7 +71,7 @@ struct Options {
   int pair = 1;            // 1 = tiles of more than 128 tokens with consecutive activation rows and K >= 2048 run on clusters of two CTAs (tcgen05.mma.cta_group::2)
   int npair = 1;           // 1 = tiles of <= 128 tokens with consecutive activation rows span two 128-row weight blocks
   int ksplit = 1;          // 1 = layouts with one MMA issuer split small tiles' K halves over two issuers
-  int decode_kernel = 1;   // 1 = token tiles of <= 32 rows (indexed, masked) use the warpgroup-per-worker kernel; 0 = never
+  int decode_kernel = 1;   // 1 = token tiles of <= 32 rows (indexed, masked) use the kernel of independent workers on mma.sync; 0 = never
   int max_stages = 0;      // 0 = as many as fit
   int grid_limit = 0;      // 0 = one CTA per SM
   int pdl = 0;             // 1 = `indexed` launches carry the programmatic stream-serialization attribute

@@ -338,21 +338,8 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem desc], kind::f16 (BF16 inputs, FP32 accumulate).
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The four K16 MMAs of one 64-wide K half in one statement: A columns a, a + 8, a + 16,
+// D[tmem] (+)= A[tmem] * B[smem desc], kind::f16 (BF16 inputs, FP32 accumulate): the four
+// K16 MMAs of one 64-wide K half in one statement, A columns a, a + 8, a + 16,
 // a + 24 of tensor memory, B descriptor advanced by 32 bytes (two 16-byte units) per K16.
 // Only the first one may start a new accumulation.  Written as one block so that the
 // operand arithmetic stays next to the instructions and, with warp-uniform inputs, in

@@ -1123,7 +1123,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const uint32_t s_off = (q >> 1) * 128u + (lane >> 2) * 16u + (q & 1) * 8u;
     StageCursor cur, acur;
     uint32_t it = 0;
-    bool ok = true;
+    uint32_t bad = 0;  // set by the first bounded wait that gives up; tested once per stage
+    const uint32_t abort_addr = ptx::smem_u32(&sh.abort_flag);
+    const uint32_t wfull0 = ptx::smem_u32(&sh.wfull[0]), wempty0 = ptx::smem_u32(&sh.wempty[0]);
+    const uint32_t aempty0 = ptx::smem_u32(&sh.aempty[0]), afull0 = ptx::smem_u32(&sh.afull[0]);
     // A stored K half is published to the MMA issuer one compute step later (after
     // the next half has been dequantised), so that the latency of the tensor-memory
     // store and of the barrier round trip hides behind ALU work.  `pending` is the
@@ -1134,10 +1137,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
+        const uint32_t full = afull0 + static_cast<uint32_t>(pending) * 8u;
+        if constexpr (kPair) {
           // `pair`: the leader's barrier counts the warps of both CTAs
-          if constexpr (kPair) ptx::mbar_arrive_cluster(ptx::smem_u32(&sh.afull[pending]) + to_leader);
-          else ptx::mbar_arrive(ptx::smem_u32(&sh.afull[pending]));
+          if (lane == 0) ptx::mbar_arrive_cluster(full + to_leader);
+        } else {
+          ptx::mbar_arrive_lane0(full, lane);
         }
         pending = -1;
       }
@@ -1166,16 +1171,15 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // Waits for the slot to be free, then stores one K half: lo to TMEM lanes 0-15 of
     // the quarter (first slab), hi to lanes 16-31 (second slab).
     auto store_half = [&](uint32_t slot, uint32_t aph, const uint32_t (&lo)[16],
-                          const uint32_t (&hi)[16]) -> bool {
-      if (!ptx::mbar_wait_warp(ptx::smem_u32(&sh.aempty[slot]), aph ^ 1u, abort_flag)) return false;
+                          const uint32_t (&hi)[16]) {
+      ptx::mbar_wait_sticky(aempty0 + slot * 8u, aph ^ 1u, abort_addr, bad);
       ptx::tc_fence_after();
       const uint32_t a_addr = tmem_base + ((q * 32u) << 16) + slot * (kAColsPerStage / 2);
       ptx::tmem_st_16x128b_x8(a_addr, lo);
       ptx::tmem_st_16x128b_x8(a_addr + (16u << 16), hi);
       pending = static_cast<int32_t>(slot);
-      return true;
     };
-    while (ok && iter.next(seg)) {
+    while (bad == 0 && iter.next(seg)) {
       const TileInfo t = decode_tile(p, sh, seg.tile, rank);
       if (!t.valid) continue;
       // This group owns the stages whose running index is `group` modulo the number
@@ -1196,10 +1200,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                           acur.advance_by(kDequantGroups, a_stages)) {
         const uint32_t a = acur.s << 1;  // half-slots a (first K half) and a + 1 (second)
         const uint32_t aph = acur.ph;
-        if (!ptx::mbar_wait_warp(ptx::smem_u32(&sh.wfull[cur.s]), cur.ph, abort_flag)) {
-          ok = false;
-          break;
-        }
+        ptx::mbar_wait_sticky(wfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
         const uint8_t* wsrc = smem_w + cur.s * kWStageBytes + w_off;
         const uint8_t* ssrc = smem_s + cur.s * kSStageBytes + s_off;
         uint2 words[4], scales[2];
@@ -1211,20 +1212,16 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         load_half(wsrc, ssrc, 1, words, scales);
         publish();  // previous stage's second half
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&sh.wempty[cur.s]));
-        if (!store_half(a, aph, lo, hi)) {
-          ok = false;
-          break;
-        }
+        ptx::mbar_arrive_lane0(wempty0 + cur.s * 8u, lane);
+        store_half(a, aph, lo, hi);
         dequant_half(words, scales, lo, hi);
         publish();  // this stage's first half
-        if (!store_half(a + 1, aph, lo, hi)) {
-          ok = false;
-          break;
-        }
+        store_half(a + 1, aph, lo, hi);
+        bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
+        if (bad != 0) break;
       }
       // `it` overshoots the segment's end by less than one stride: bring the cursor back.
-      if (ok) {
+      if (bad == 0) {
         const uint32_t over = it - it_end;
         it = it_end;
         cur.advance_by(w_stages - over, w_stages);
@@ -1234,10 +1231,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       }
     }
     publish();
-    if (!ok && lane == 0) {
-      sh.abort_flag = 1;
-      if (p.status) atomicOr(p.status, kStatusDequantTimeout);
-    }
+    if (bad != 0 && lane == 0 && p.status) atomicOr(p.status, kStatusDequantTimeout);
   } else {
     // -------------------------------------------------------------- epilogue --
     // Four warps, one per tensor-memory lane quarter; with `tiled_roles` a second group of
@@ -1322,9 +1316,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         // A whole tile on eight epilogue warps: the warp's share of the accumulators (at most
         // eight chunks of 16 columns) is read and rounded first, the accumulators go back to
         // the issuers, and only then are the rows written.  Accumulators of this size are
-        // single-buffered: what is left between two tiles is the reading alone.  (contiguous,
-        // 8192 uneven rows: gate_up 521 -> 513 us, down, 16 stages per tile, 388 -> 334 us;
-        // 24000 rows: 1235 / 891 -> 1139 / 839 us.)
+        // single-buffered: what is left between two tiles is the reading alone.
         constexpr int kChunks = 8;
         uint32_t held[kChunks][8];
         const int32_t first = static_cast<int32_t>(egroup) * 16;

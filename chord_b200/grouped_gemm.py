@@ -2,7 +2,7 @@
 chord_kernels/ops.py:49-90 and chord_kernels/operator/grouped/api.py:116-271.
 
 The reference implements these for SM90 only (WGMMA); here they run on the same
-sm_100a tcgen05 kernel as ``indexed`` with a different tile scheduler."""
+sm_100a kernels as ``indexed`` with a different tile scheduler."""
 
 from __future__ import annotations
 

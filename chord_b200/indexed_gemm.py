@@ -1,6 +1,6 @@
 """``indexed`` / ``indexed_block_m``: the routed (``moe_align_block_size``) W4A16
 MoE GEMM, same interface as chord_kernels/ops.py:8-46 and
-chord_kernels/operator/api.py:300-409, on the sm_100a tcgen05 kernel."""
+chord_kernels/operator/api.py:300-409, on the sm_100a kernels."""
 
 from __future__ import annotations
 

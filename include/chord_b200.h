@@ -70,7 +70,7 @@ const char* chord_b200_version(void);
  *                     (single-block experts, the last block of an odd run) on 128-token
  *                     tiles; 0 off
  *   "decode_kernel"   1 (default) token tiles of at most 32 rows (indexed, masked) run
- *                     the warpgroup-per-worker kernel; 0 always the general kernel
+ *                     the kernel of independent workers on mma.sync; 0 always the general kernel
  *   "max_stages"      0 as many shared-memory stages as fit (default), else a cap
  *   "grid_limit"      0 one CTA per SM (default), else at most this many CTAs
  *   "pdl"             1 launches of `indexed` and the SiLU*mul kernels carry the

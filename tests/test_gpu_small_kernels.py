@@ -1,0 +1,74 @@
+"""Edges of the kernels either side of the GEMMs: where the alignment kernel changes its shape
+(4096 ids, counters beyond 160 KB, more than one batch of loads), remainders and alignment of
+the packer, row lengths of SiLU*mul."""
+
+import pytest
+import torch
+
+from oracle import w4a16_oracle as O
+from tests.cases import make_weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("numel", [1, 511, 4095, 4096, 4097, 16385, 40001])
+@pytest.mark.parametrize("experts,total,base", [(48, 384, 96), (1, 2, 1), (1240, 1240, 0), (1241, 1300, 7), (2048, 2048, 0)])
+def test_alignment_shapes(device, numel, experts, total, base):
+    import chord_b200
+
+    g = torch.Generator().manual_seed(numel + experts)
+    topk = torch.randint(0, total, (numel, 1), generator=g, dtype=torch.int32)
+    s, e, p = chord_b200.moe_align_block_size(topk.to(device), 16, experts, expert_base=base)
+    rs, re, rp = O.align_routing_blocks(topk, 16, experts, base)
+    count = int(p.item())
+    assert count == int(rp)
+    assert torch.equal(s.cpu()[:count], rs)
+    assert torch.equal(e.cpu()[: count // 16], re)
+
+
+def test_alignment_ids_outside_every_range(device):
+    import chord_b200
+
+    ids = torch.tensor([[-2**31, 2**31 - 1, -1, 5, 7, 8, 4]], dtype=torch.int32)
+    s, e, p = chord_b200.moe_align_block_size(ids.to(device), 8, 3, expert_base=5)  # experts 5, 6, 7
+    assert int(p.item()) == 16
+    assert s.cpu()[:16].tolist() == [3] + [7] * 7 + [4] + [7] * 7
+    assert e.cpu()[:2].tolist() == [0, 2]
+
+
+@pytest.mark.parametrize("k", [64, 448, 512, 576, 1088])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_packer_remainders_and_scale_alignment(device, k, offset):
+    import chord_b200
+
+    codes, scale = make_weights(2, 256, k, seed=k + offset)
+    buffer = torch.zeros(scale.numel() + offset, dtype=torch.bfloat16, device=device)
+    view = buffer[offset:].view(scale.shape)  # 2-, 4- or 16-byte aligned
+    view.copy_(scale)
+    words = torch.from_numpy(O.pack_checkpoint_uint4(codes.numpy())).to(device)
+    want = torch.from_numpy(O.repack_closed_form(codes.numpy()))
+    for w in (chord_b200.pack_w4a16(words, view, packed=True), chord_b200.pack_w4a16(codes.to(device), view)):
+        assert torch.equal(w.packed.cpu(), want)
+        assert torch.equal(w.scale.cpu().view(torch.int16), O.permute_scale(scale).view(torch.int16))
+
+
+@pytest.mark.parametrize("rows,inter", [(1, 8), (300, 8), (7, 24), (33, 264), (5, 2048), (3, 2056)])
+def test_silu_mul_row_lengths(device, rows, inter):
+    """FP32 arithmetic within a few units of 2^-21, then one rounding to BF16 (2^-8 at most)."""
+    import chord_b200
+
+    x = torch.randn((rows, 2 * inter), generator=torch.Generator().manual_seed(inter)).to(torch.bfloat16)
+    got = chord_b200.silu_mul(x.to(device)).cpu().double()
+    gate, up = x[:, :inter].double(), x[:, inter:].double()
+    want = gate / (1 + torch.exp(-gate)) * up
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -18)).all())
+
+
+def test_silu_mul_extreme_gates(device):
+    import chord_b200
+
+    gate = torch.tensor([float("inf"), float("-inf"), float("nan"), 3e38, -3e38, -88.5, -87.0, 0.0], dtype=torch.bfloat16)
+    x = torch.cat([gate, torch.ones_like(gate)]).view(1, 16)
+    got = chord_b200.silu_mul(x.to(device)).cpu().float()[0]
+    assert got[0] == float("inf") and torch.isnan(got[1]) and torch.isnan(got[2])
+    assert got[3] > 2.9e38 and got[4] == 0 and -1e-35 < got[5] <= 0 and -2e-35 < got[6] < 0 and got[7] == 0
