@@ -72,3 +72,25 @@ def test_silu_mul_extreme_gates(device):
     got = chord_b200.silu_mul(x.to(device)).cpu().float()[0]
     assert got[0] == float("inf") and torch.isnan(got[1]) and torch.isnan(got[2])
     assert got[3] > 2.9e38 and got[4] == 0 and -1e-35 < got[5] <= 0 and -2e-35 < got[6] < 0 and got[7] == 0
+
+
+@pytest.mark.parametrize("expected_m,n,k", [(120, 256, 2048), (121, 256, 2048), (144, 512, 2112), (130, 384, 2048),
+                                            (130, 256, 1984)])
+def test_masked_tile_choice(device, expected_m, n, k):
+    """Both sides of the line between 128- and 256-row tiles; counts below, at and above both."""
+    import chord_b200
+
+    counts, max_m = (0, 1, 127, 128, 129, 200, 256, 300), 300
+    codes, scale = make_weights(len(counts), n, k, seed=k + expected_m)
+    w = chord_b200.pack_w4a16(codes.to(device), scale.to(device))
+    x = torch.randn((len(counts), max_m, k), generator=torch.Generator().manual_seed(k)).to(torch.bfloat16)
+    out = torch.full((len(counts) * max_m, n), -7.0, dtype=torch.bfloat16, device=device)
+    chord_b200.masked(x.to(device), w, torch.tensor(counts, dtype=torch.int32, device=device), expected_m, outputs=out)
+    out = out.cpu().view(len(counts), max_m, n)
+    wd = ((codes - 8).to(torch.bfloat16) * scale.repeat_interleave(32, 2)).float()
+    for g, c in enumerate(counts):
+        ref = x[g, :c].float() @ wd[g].T
+        # FP32 sums in two orders (2^-22 of the absolute products per term's depth), one BF16 rounding
+        bound = 2.0 ** -17 * (x[g, :c].float().abs() @ wd[g].abs().T)
+        assert bool(((out[g, :c].float() - ref).abs() <= 1.01 * (ref.abs() * 2.0 ** -8 + bound)).all())
+        assert bool((out[g, c:] == -7.0).all())
