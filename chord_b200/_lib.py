@@ -43,6 +43,7 @@ SIGNATURES = {
     "chord_b200_indexed_workspace_bytes": (_i64, [_i64, _i64, _i64]),
     "chord_b200_gemm_lock_words": (_int, []),
     "chord_b200_schedule_segments": (_i64, [_i64, _i64, _i64, _i64, _ptr, _i64]),
+    "chord_b200_decode_schedule_segments": (_i64, [_i64, _i64, _int, _i64, _i64, _ptr, _i64]),
     "chord_b200_indexed": (_int, [_ptr, _ptr, _ptr, _ptr, _i64, _ptr, _i64, _ptr, _ptr, _ptr, _i64,
                                   _ptr, _i64, _ptr, _i64, _i64, _i64, _i64, _i64, _i64, _ptr]),
     "chord_b200_indexed_rows": (_int, [_ptr, _ptr, _ptr, _ptr, _i64, _ptr, _i64, _ptr, _ptr, _ptr, _i64,

@@ -614,16 +614,11 @@ int chord_b200_gemm_lock_words(void) {
   return chord::decode_workers(chord::grid_size(dev));
 }
 
-int64_t chord_b200_schedule_segments(int64_t tiles, int64_t k, int64_t grid, int64_t cta,
-                                     int32_t* out, int64_t capacity) {
-  if (tiles < 0 || k <= 0 || k % 64 || grid <= 0 || cta < 0 || cta >= grid ||
-      tiles > (1ll << 30)) {
-    chord::fail(chord::kInvalidArgument, "bad schedule query");
-    return -1;
-  }
+static int64_t walk_schedule(int64_t tiles, int64_t k_steps, int64_t grid, int64_t cta, bool decode,
+                             int32_t* out, int64_t capacity) {
   chord::SegmentIterator it;
-  it.init(static_cast<int32_t>(tiles), static_cast<int32_t>((k + chord::kBlockK - 1) / chord::kBlockK),
-          static_cast<int32_t>(grid), static_cast<int32_t>(cta));
+  it.init(static_cast<int32_t>(tiles), static_cast<int32_t>(k_steps), static_cast<int32_t>(grid),
+          static_cast<int32_t>(cta), decode);
   chord::Segment seg;
   int64_t count = 0;
   while (it.next(seg)) {
@@ -638,6 +633,28 @@ int64_t chord_b200_schedule_segments(int64_t tiles, int64_t k, int64_t grid, int
     ++count;
   }
   return count;
+}
+
+static bool schedule_query_ok(int64_t tiles, int64_t k, int64_t grid, int64_t cta) {
+  if (tiles >= 0 && k > 0 && k % 64 == 0 && k < (1ll << 31) && grid > 0 && cta >= 0 && cta < grid &&
+      tiles <= (1ll << 30)) {
+    return true;
+  }
+  chord::fail(chord::kInvalidArgument, "bad schedule query");
+  return false;
+}
+
+int64_t chord_b200_schedule_segments(int64_t tiles, int64_t k, int64_t grid, int64_t cta,
+                                     int32_t* out, int64_t capacity) {
+  if (!schedule_query_ok(tiles, k, grid, cta)) return -1;
+  return walk_schedule(tiles, (k + chord::kBlockK - 1) / chord::kBlockK, grid, cta, false, out, capacity);
+}
+
+int64_t chord_b200_decode_schedule_segments(int64_t tiles, int64_t k, int fuse_silu, int64_t workers,
+                                            int64_t worker, int32_t* out, int64_t capacity) {
+  if (!schedule_query_ok(tiles, k, workers, worker)) return -1;
+  const int64_t steps = (k + chord::kDecStageK - 1) / chord::kDecStageK << (fuse_silu != 0);
+  return walk_schedule(tiles, steps, workers, worker, true, out, capacity);
 }
 
 static int indexed_launch(const void* x, const int32_t* packed, const void* scale,

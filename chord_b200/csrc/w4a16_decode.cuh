@@ -44,10 +44,6 @@ constexpr int kDecMaxStages = 6;
 constexpr int kDecMaxTokens = 32;
 constexpr int kDecWorkers = 4;                        // workers per CTA
 constexpr int kDecThreads = 32 * (kDecWorkers + 4 * kDecWorkers);  // feeders, computing warps
-// Shortest stream-K slice in K blocks (a fused gate_up tile has two stages per K block).
-// 8 experts of 1024 x 512, 64 tokens (four blocks per tile): 12.8 us with slices of eight,
-// 8.7 us with four; longer K: no difference.
-constexpr int kDecMinSlice = 4;
 constexpr int kDecPitch = 40;  // BF16 per token row of the epilogue buffer: 32 rows, padded against bank conflicts
 
 struct __align__(16) DecodeWorkerShared {
@@ -120,8 +116,8 @@ struct StepStream {
   int32_t kb;
   bool live;
 
-  __device__ void init(int32_t tiles, int32_t k_steps, int32_t workers, int32_t worker, int32_t min_slice) {
-    iter.init(tiles, k_steps, workers, worker, min_slice);
+  __device__ void init(int32_t tiles, int32_t k_steps, int32_t workers, int32_t worker) {
+    iter.init(tiles, k_steps, workers, worker, true);
     live = false;
     kb = 0;
   }
@@ -480,7 +476,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       dst_off[b] = r * 128u + ((piece ^ (r & 7u)) << 4);
     }
     StepStream steps;
-    steps.init(tiles, k_steps, workers, worker_id, kDecMinSlice << fuse);
+    steps.init(tiles, k_steps, workers, worker_id);
     StageCursor cur;
     uint32_t issued = 0;  // stages handed to the TMA so far, up to the ring's depth
     uint32_t bad = 0;
@@ -561,7 +557,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     ring.bytes = worker_bytes;
     ring.abort_addr = abort_addr;
     SegmentIterator iter;
-    iter.init(tiles, k_steps, workers, worker_id, kDecMinSlice << fuse);
+    iter.init(tiles, k_steps, workers, worker_id, true);
     Segment seg;
     while (iter.next(seg)) {
       const TileInfo t = decode_tile_small(p, sh.group_prefix, seg.tile);

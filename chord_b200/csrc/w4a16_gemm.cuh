@@ -167,6 +167,10 @@ struct Segment {
   int32_t peer;    // owner: number of contributors; contributor: owner CTA
 };
 
+// Shortest stream-K slice in K steps.  A finer split costs more in partial sums and per-slice
+// set-up than the extra parallelism returns.
+constexpr int32_t kMinSlice = 8;
+
 // Enumerates the work of one CTA; every warp role walks the same sequence.
 struct SegmentIterator {
   int32_t grid, cta, ki;
@@ -174,24 +178,29 @@ struct SegmentIterator {
   int64_t units, u0, u1;
   int32_t geff;
 
+  // `whole_short_tiles` (decode kernels, whose workers commonly outnumber the tiles): tiles
+  // shorter than kMinSlice are dealt out whole instead of several to a worker (8 experts of 1024 x
+  // 512, four steps per tile: 12.8 us with slices of eight, 8.7 us with whole tiles).  Longer tiles
+  // keep slices of eight: with four, 64 experts of 1024 x 1024 (512 tiles of eight steps, 592
+  // workers) were cut up instead of taken whole, 17.9 us against 14.0 us with 1 row per expert.
   __host__ __device__ void init(int32_t tiles, int32_t k_iters, int32_t grid_, int32_t cta_,
-                                int32_t min_slice = 8) {
+                                bool whole_short_tiles = false) {
     grid = grid_;
     cta = cta_;
     ki = k_iters;
     dp_waves = tiles / grid;
     int32_t sk_tiles = tiles - dp_waves * grid;
-    // A short tail would be cut into slivers: fold one full wave into it.
-    if (dp_waves > 0 && sk_tiles > 0 && static_cast<int64_t>(sk_tiles) * ki < 8ll * grid) {
+    // A tail of less than kMinSlice steps per CTA would be cut into slivers: fold one full wave into it.
+    if (dp_waves > 0 && sk_tiles > 0 && static_cast<int64_t>(sk_tiles) * ki < static_cast<int64_t>(kMinSlice) * grid) {
       dp_waves -= 1;
       sk_tiles += grid;
     }
     dp_tiles = dp_waves * grid;
     wave = 0;
     units = static_cast<int64_t>(sk_tiles) * ki;
-    // No slice shorter than `min_slice` k-blocks (unless the whole tail is): a finer split
-    // costs more in partial sums and per-slice set-up than the extra parallelism returns.
-    const int64_t slices = units / min_slice > 0 ? units / min_slice : (units > 0 ? 1 : 0);
+    // No slice shorter than kMinSlice (unless the whole tail is).
+    int64_t slices = units / kMinSlice > 0 ? units / kMinSlice : (units > 0 ? 1 : 0);
+    if (whole_short_tiles && ki < kMinSlice) slices = sk_tiles;
     geff = slices < grid ? static_cast<int32_t>(slices) : grid;
     if (cta < geff) {
       u0 = cta * units / geff;

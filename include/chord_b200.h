@@ -135,6 +135,12 @@ int chord_b200_gemm_lock_words(void);
 int64_t chord_b200_schedule_segments(int64_t tiles, int64_t k, int64_t grid, int64_t cta,
                                      int32_t* out, int64_t capacity);
 
+/* The same for worker `worker` of a launch of the decode kernel (token tiles of at most 32
+ * rows) with `workers` workers, four per CTA.  Its K steps are 128 wide; with fuse_silu != 0
+ * a tile has two per K block (gate, up). */
+int64_t chord_b200_decode_schedule_segments(int64_t tiles, int64_t k, int fuse_silu, int64_t workers,
+                                            int64_t worker, int32_t* out, int64_t capacity);
+
 /* ---- indexed GEMM: replaces launch_kernel (launcher.cpp:52-158) -------------
  * out[id, :] = x[id / top_k, :] . dequant(W[expert_ids[block of id]])^T for every
  * id < m * top_k found in sorted_ids[0 .. *num_tokens_padded).

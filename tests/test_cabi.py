@@ -136,6 +136,31 @@ def test_schedule_slices_are_not_slivers(native_lib, tiles, k, grid):
     assert busy <= max(1, grid)
 
 
+@pytest.mark.parametrize("tiles,k,fuse", [(32, 7168, 0), (56, 2048, 0), (512, 1024, 0), (64, 512, 0), (600, 512, 0),
+                                          (9, 192, 0), (1, 64, 0), (1536, 7168, 0), (16, 128, 1), (700, 384, 1),
+                                          (64, 2048, 1)])
+@pytest.mark.parametrize("workers", [592, 20])
+def test_decode_schedule(native_lib, tiles, k, fuse, workers):
+    """Every step once; tiles are taken whole where the workers outnumber them and a tile has at
+    most eight steps, and otherwise cut into slices of at least eight (the split of `tiles` over
+    `workers` that the order of the FP32 sums follows)."""
+    steps = ((k + 127) // 128) << fuse
+    cover = np.zeros((tiles, steps), dtype=np.int64)
+    for worker in range(workers):
+        buf = (ctypes.c_int32 * 5000)()
+        n = native_lib.chord_b200_decode_schedule_segments(tiles, k, fuse, workers, worker,
+                                                           ctypes.cast(buf, ctypes.c_void_p), 1000)
+        segs = np.frombuffer(buf, dtype=np.int32)[: 5 * n].reshape(n, 5)
+        for tile, kb, ke, kind, _ in segs:
+            cover[tile, kb:ke] += 1
+            assert (kind == 0) == (kb == 0 and ke == steps)
+            if tiles <= workers and steps <= 8:
+                assert kind == 0
+        work = sum(int(s[2] - s[1]) for s in segs)
+        assert work == 0 or work >= min(8, steps)
+    assert (cover == 1).all()
+
+
 def test_schedule_rejects_bad_queries(native_lib):
     assert native_lib.chord_b200_schedule_segments(10, 100, 148, 0, None, 0) < 0
     assert native_lib.chord_b200_schedule_segments(10, 128, 148, 148, None, 0) < 0
