@@ -52,7 +52,8 @@ def test_packer_remainders_and_scale_alignment(device, k, offset):
         assert torch.equal(w.scale.cpu().view(torch.int16), O.permute_scale(scale).view(torch.int16))
 
 
-@pytest.mark.parametrize("rows,inter", [(1, 8), (300, 8), (7, 24), (33, 264), (5, 2048), (3, 2056)])
+@pytest.mark.parametrize("rows,inter", [(1, 8), (300, 8), (7, 24), (33, 264), (5, 2048), (3, 2056),
+                                        (2, 32776)])
 def test_silu_mul_row_lengths(device, rows, inter):
     """FP32 arithmetic within a few units of 2^-21, then one rounding to BF16 (2^-8 at most)."""
     import chord_b200
@@ -62,6 +63,44 @@ def test_silu_mul_row_lengths(device, rows, inter):
     gate, up = x[:, :inter].double(), x[:, inter:].double()
     want = gate / (1 + torch.exp(-gate)) * up
     assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -18)).all())
+
+
+@pytest.mark.parametrize("block_m", [16, 64])
+def test_silu_mul_is_the_fused_epilogue(device, block_m):
+    """One function, wherever it is computed: with weights that pick single activations the FP32
+    accumulators of gate_up hold BF16 values exactly, and the fused epilogue (an IEEE quotient in
+    FP32, one rounding) and the separate kernel give the same bits.  A quotient off by a unit in
+    the last place of FP32 changes about one BF16 result in 2^16."""
+    import chord_b200
+    from chord_b200.indexed_gemm import indexed_gate_up_silu
+
+    n, tokens = 256, 32768
+    codes = torch.full((1, n, n), 8, dtype=torch.int32)
+    codes[0].fill_diagonal_(9)
+    w = chord_b200.pack_w4a16(codes.to(device), torch.ones((1, n, n // 32), dtype=torch.bfloat16, device=device))
+    x = torch.randn((tokens, n), generator=torch.Generator().manual_seed(3)).mul_(3).to(torch.bfloat16).to(device)
+    routing = (torch.arange(tokens, dtype=torch.int32, device=device),
+               torch.zeros(tokens // block_m, dtype=torch.int32, device=device),
+               torch.tensor([tokens], dtype=torch.int32, device=device))
+    gate_up = chord_b200.indexed(x, w, *routing, 1, block_m=block_m)
+    assert torch.equal(gate_up, x)
+    fused = indexed_gate_up_silu(x, w, *routing, 1, block_m=block_m)
+    assert torch.equal(chord_b200.silu_mul(gate_up), fused)
+
+
+def test_silu_mul_of_zero_gates(device):
+    """Vectors of zero gates keep the sign of the product and what 0 * inf and 0 * nan give."""
+    import chord_b200
+
+    up = torch.tensor([1.0, -1.0, 0.0, -0.0, float("inf"), float("nan"), 1e-40, -3e38], dtype=torch.bfloat16)
+    for gates in ([0.0] * 8, [-0.0] * 8, [0.0, -0.0] * 4, [0.0] * 7 + [2.0]):
+        gate = torch.tensor(gates, dtype=torch.bfloat16)
+        got = chord_b200.silu_mul(torch.cat([gate, up]).view(1, 16).to(device)).cpu()[0].float()
+        want = torch.nn.functional.silu(gate.float()) * up.float()
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        keep = ~torch.isnan(want)
+        assert torch.equal(torch.signbit(got[keep]), torch.signbit(want[keep]))
+        assert torch.allclose(got[keep], want[keep], rtol=2.0 ** -8, atol=0)
 
 
 def test_silu_mul_extreme_gates(device):
