@@ -69,16 +69,20 @@ def test_silu_mul_row_lengths(device, rows, inter):
 def test_silu_mul_is_the_fused_epilogue(device, block_m):
     """One function, wherever it is computed: with weights that pick single activations the FP32
     accumulators of gate_up hold BF16 values exactly, and the fused epilogue (an IEEE quotient in
-    FP32, one rounding) and the separate kernel give the same bits.  A quotient off by a unit in
-    the last place of FP32 changes about one BF16 result in 2^16."""
+    FP32, one rounding) and the separate kernel give the same bits.  Half of the gates are the two
+    BF16 values whose quotient lies so close to a rounding boundary of some products that
+    v * reciprocal(1 + e^-v) lands on the other side."""
     import chord_b200
     from chord_b200.indexed_gemm import indexed_gate_up_silu
 
-    n, tokens = 256, 32768
+    n, tokens = 256, 8192
     codes = torch.full((1, n, n), 8, dtype=torch.int32)
     codes[0].fill_diagonal_(9)
     w = chord_b200.pack_w4a16(codes.to(device), torch.ones((1, n, n // 32), dtype=torch.bfloat16, device=device))
-    x = torch.randn((tokens, n), generator=torch.Generator().manual_seed(3)).mul_(3).to(torch.bfloat16).to(device)
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn((tokens, n), generator=g).sign_() * torch.exp(torch.rand((tokens, n), generator=g) * 12 - 8)
+    x[::4, :n // 2], x[1::4, :n // 2] = -15.0, 0.0004444122314453125
+    x = x.to(torch.bfloat16).to(device)
     routing = (torch.arange(tokens, dtype=torch.int32, device=device),
                torch.zeros(tokens // block_m, dtype=torch.int32, device=device),
                torch.tensor([tokens], dtype=torch.int32, device=device))
