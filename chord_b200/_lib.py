@@ -39,6 +39,7 @@ SIGNATURES = {
     "chord_b200_permute_scale": (_int, [_ptr, _ptr, _i64, _i64, _i64, _ptr]),
     "chord_b200_indexed_block_m": (_int, [_i64, _i64, _i64, _i64]),
     "chord_b200_masked_tile_m": (_int, [_i64]),
+    "chord_b200_masked_tile_rows": (_int, [_i64, _i64, _i64, _i64]),
     "chord_b200_gemm_workspace_bytes": (_i64, [_i64]),
     "chord_b200_indexed_workspace_bytes": (_i64, [_i64, _i64, _i64]),
     "chord_b200_gemm_lock_words": (_int, []),

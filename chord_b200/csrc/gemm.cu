@@ -245,6 +245,13 @@ bool pair_applies(int mma_n, int n, int k) {
   return options().pair != 0 && mma_n > 128 && k >= 2048 && (n / kBlockN) % 2 == 0;
 }
 
+// Whether the current device keeps CTA pairs of the general kernel resident at all.
+bool pairs_resident(const DeviceInfo& dev) {
+  if (grid_size(dev) < 2) return false;
+  const size_t optin = static_cast<size_t>(dev.max_smem_optin);
+  return (options().dequant_groups == 4 ? resident_pairs<4>(optin) : resident_pairs<2>(optin)) >= 1;
+}
+
 bool pregather_applies(int mma_n) { return options().pregather != 0 && mma_n >= 64; }
 
 // Token tiles of at most 32 rows (indexed, masked) have a kernel of their own, in which
@@ -557,15 +564,33 @@ int chord_b200_indexed_block_m(int64_t n, int64_t k, int64_t num_experts, int64_
 
 int chord_b200_masked_tile_m(int64_t expected_m) {
   // A group with more rows than the tile costs a second pass over its weights, so the
-  // tile leaves room for the spread around the expected count (measured on 24 groups of
-  // 4096 x 7168 with Poisson row counts: at 32 expected rows 64-token tiles take 170 us
-  // against 200 us for 32-token tiles, at 64 rows 128-token tiles 182 us against 236 us,
-  // at 128 rows 128-token tiles 254 us against 279 us for 256-token tiles on CTA pairs,
-  // at 200 rows 350 us against 295 us).
+  // tile leaves room for the spread around the expected count.
   if (expected_m <= 8) return 16;
   if (expected_m <= 20) return 32;
   if (expected_m <= 48) return 64;
   if (expected_m <= 144) return 128;
+  return 256;
+}
+
+// From an expected 121 rows on many groups exceed a 128-row tile and would pay a second pass
+// over their weights: 256-row tiles instead, where those run on CTA pairs.  128- against 256-row
+// tiles, us, weights from HBM:
+//   24 groups, Poisson counts      4096 x 7168   7168 x 2048   512 x 2048
+//     112 expected                 181 / 209     119 / 106     29 / 26
+//     121                          218 / 199     124 / 106     28 / 27
+//     128                          281 / 200     156 / 112     33 / 28
+//     144                          285 / 212     173 / 116     37 / 29
+//   128 rows in every group        174 / 193     117 / 109     28 / 26
+//     16 (expected_m far too high) 132 / 157     86 / 95       20 / 19
+int chord_b200_masked_tile_rows(int64_t expected_m, int64_t max_m, int64_t n, int64_t k) {
+  chord::OptionsReadLock options_guard(chord::options_mutex());
+  const int tile_m = chord_b200_masked_tile_m(expected_m);
+  if (tile_m != 128 || expected_m <= 120 || max_m <= 128 || n <= 0 || n > INT32_MAX || k > INT32_MAX ||
+      !chord::pair_applies(256, static_cast<int>(n), static_cast<int>(k))) {
+    return tile_m;
+  }
+  chord::DeviceInfo dev;  // (without a device the answer is that of a whole B200)
+  if (chord::current_device_info(&dev) == chord::kOk && !chord::pairs_resident(dev)) return tile_m;
   return 256;
 }
 

@@ -6,10 +6,12 @@ sm_100a kernels as ``indexed`` with a different tile scheduler."""
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _checks, _lib
-from .indexed_gemm import gemm_scratch, status_word
+from .indexed_gemm import _device_index, gemm_scratch, status_word
 from .packing import PreparedWeight
 
 
@@ -31,17 +33,12 @@ def masked_tile_m(expected_m: int) -> int:
     return int(_lib.native().chord_b200_masked_tile_m(expected_m))
 
 
-def _tile_rows(expected_m: int, max_m: int, n: int, k: int) -> int:
-    """Token tile of a masked launch.  From an expected 121 rows on many groups exceed a
-    128-row tile and would pay a second pass over their weights: where 256-row tiles run on
-    CTA pairs (two whole weight blocks, K >= 2048) those are used instead.  Measured, 24
-    groups with Poisson counts, gate_up [4096, 7168] + down [7168, 2048], 128- against
-    256-row tiles: expected 112 rows 274 / 301 us, 120 rows 302 / 304, 128 rows 355 / 317,
-    144 rows 435 / 340."""
-    tile_m = masked_tile_m(expected_m)
-    if tile_m == 128 and expected_m > 120 and max_m > 128 and n % 256 == 0 and k >= 2048:
-        return 256
-    return tile_m
+@functools.lru_cache(maxsize=256)
+def _tile_rows(device_index: int, expected_m: int, max_m: int, n: int, k: int, options_epoch: int) -> int:
+    """Token tile of a masked launch, asked of the library once per shape, device and option
+    setting (the current device must be ``device_index``)."""
+    del device_index, options_epoch  # cache keys only
+    return int(_lib.load().chord_b200_masked_tile_rows(expected_m, max_m, n, k))
 
 
 def w4a16_masked(
@@ -85,9 +82,9 @@ def w4a16_masked(
         outputs = torch.empty((groups * max_m, weight.n), dtype=torch.bfloat16, device=device)
     else:
         _checks.bf16_output(outputs, (groups * max_m, weight.n), device, exact_shape=False)
-    tile_m = _tile_rows(expected_m, max_m, weight.n, weight.k)
     lib = _lib.native()
     with _lib.on_device(device):
+        tile_m = _tile_rows(_device_index(device), expected_m, max_m, weight.n, weight.k, _lib.options_epoch())
         locks, workspace, ws_bytes = gemm_scratch(device, tile_m, None)
         _lib.check(lib.chord_b200_masked(
             grouped.data_ptr(), weight.packed.data_ptr(), weight.scale.data_ptr(),

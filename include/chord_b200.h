@@ -103,9 +103,12 @@ int chord_b200_permute_scale(const void* in, void* out, int64_t num_experts, int
  * tuning.py:512-554).  Always a multiple of 8. */
 int chord_b200_indexed_block_m(int64_t n, int64_t k, int64_t num_experts, int64_t routed_m);
 
-/* Token-tile size the masked kernel uses for `expected_m` (replaces
- * _w4a16_masked_bm, chord_kernels/operator/grouped/heuristics.py:58-72). */
+/* Token-tile size for `expected_m` rows per group where nothing else is known (replaces
+ * _w4a16_masked_bm, chord_kernels/operator/grouped/heuristics.py:58-72), and the one
+ * `masked` uses for groups of up to `max_m` rows and an N x K weight on the current device
+ * with the present options: larger where CTA pairs (option "pair") make that pay. */
 int chord_b200_masked_tile_m(int64_t expected_m);
+int chord_b200_masked_tile_rows(int64_t expected_m, int64_t max_m, int64_t n, int64_t k);
 
 /* Bytes of FP32 stream-K scratch a GEMM launch with this token tile needs on
  * the current device (the reference allocates it per launch inside its

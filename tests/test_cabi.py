@@ -8,6 +8,7 @@ from pathlib import Path
 
 import numpy as np
 import pytest
+import torch
 
 ROOT = Path(__file__).resolve().parents[1]
 
@@ -159,6 +160,28 @@ def test_decode_schedule(native_lib, tiles, k, fuse, workers):
         work = sum(int(s[2] - s[1]) for s in segs)
         assert work == 0 or work >= min(8, steps)
     assert (cover == 1).all()
+
+
+def test_masked_tile_rows(native_lib):
+    """256-row tiles from an expected 121 rows on, and only where they run on CTA pairs."""
+    from chord_b200 import _lib
+
+    tile = native_lib.chord_b200_masked_tile_rows
+    assert [tile(m, 256, 4096, 7168) for m in (1, 8, 9, 20, 21, 48, 49, 120, 121, 144, 145, 300)] == \
+        [16, 16, 32, 32, 64, 64, 128, 128, 256, 256, 256, 256]
+    assert tile(130, 128, 4096, 7168) == 128           # no group can exceed 128 rows
+    assert tile(130, 129, 4096, 2048) == 256
+    assert tile(130, 256, 4096, 1984) == 128           # K too short for pairs
+    assert tile(130, 256, 384, 7168) == 128            # an odd number of weight blocks
+    for name in ("pair", "grid_limit"):
+        _lib.set_option(name, {"pair": 0, "grid_limit": 1}[name])
+        try:
+            if name == "pair" or torch.cuda.is_available():  # the grid is the device's
+                assert tile(130, 256, 4096, 7168) == 128
+        finally:
+            _lib.set_option(name, {"pair": 1, "grid_limit": 0}[name])
+    # without anything known about the weight the tile that needs no pairs
+    assert [native_lib.chord_b200_masked_tile_m(m) for m in (120, 121, 144, 145)] == [128, 128, 128, 256]
 
 
 def test_schedule_rejects_bad_queries(native_lib):
