@@ -105,7 +105,8 @@ def load() -> ctypes.CDLL:
 
 
 def native():
-    """The entry points for calls with plain integer arguments (addresses included): through
+    """The entry points for calls with plain integer arguments (addresses included; None is
+    the null pointer): through
     the ``_call`` extension module where it was built, otherwise the ctypes functions of
     :func:`load`.  ctypes spends 4.5 us on converting the 21 arguments of ``indexed``, the
     module less than 1 us; a pass of four calls on a small layer goes from 71 to 47 us with this and
@@ -117,7 +118,8 @@ def native():
         for name, (restype, argtypes) in SIGNATURES.items():
             fn = getattr(lib, name)
             if _call is not None and restype is _int and ctypes.c_char_p not in argtypes:
-                fn = functools.partial(_call.call, ctypes.cast(fn, ctypes.c_void_p).value)
+                signature = "".join("p" if t is _ptr else "i" for t in argtypes)
+                fn = functools.partial(_call.call, ctypes.cast(fn, ctypes.c_void_p).value, signature)
             functions[name] = fn
         _NATIVE = SimpleNamespace(**functions)
     return _NATIVE

@@ -14,6 +14,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from pathlib import Path
 
 PACKAGE_DIR = Path(__file__).resolve().parent
@@ -37,7 +38,26 @@ def _newest_source_mtime() -> float:
 
 
 def is_fresh() -> bool:
-    return LIB_PATH.exists() and LIB_PATH.stat().st_mtime >= _newest_source_mtime()
+    return LIB_PATH.exists() and LIB_PATH.stat().st_mtime >= _newest_source_mtime() and _call_module_is_fresh()
+
+
+def _call_module_path() -> Path:
+    return PACKAGE_DIR / ("_call" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _call_compiler() -> list[str] | None:
+    """What compiles the `_call` module, or None where that cannot be done here."""
+    headers = Path(sysconfig.get_paths()["include"])
+    gcc = shutil.which(os.environ.get("CC", "gcc"))
+    return [gcc, f"-I{headers}"] if gcc is not None and (headers / "Python.h").exists() else None
+
+
+def _call_module_is_fresh() -> bool:
+    """Up to date, or not to be had here (the library is then called through ctypes)."""
+    path = _call_module_path()
+    if path.exists():
+        return path.stat().st_mtime >= (CSRC / "pycall.c").stat().st_mtime
+    return _call_compiler() is None
 
 
 def _compile(nvcc: str, src: str, obj_dir: Path, verbose: bool) -> Path:
@@ -55,21 +75,22 @@ def _compile(nvcc: str, src: str, obj_dir: Path, verbose: bool) -> Path:
     return obj
 
 
-def _build_call_module(verbose: bool) -> None:
+def _build_call_module() -> None:
     """The optional ``_call`` extension module (csrc/pycall.c); without Python's headers or a C
-    compiler the library is called through ctypes instead."""
-    headers = Path(sysconfig.get_paths()["include"])
-    gcc = shutil.which(os.environ.get("CC", "gcc"))
-    if gcc is None or not (headers / "Python.h").exists():
-        return
-    out = PACKAGE_DIR / ("_call" + sysconfig.get_config_var("EXT_SUFFIX"))
-    tmp = out.with_suffix(".tmp")
-    cmd = [gcc, "-O2", "-Wall", "-fPIC", "-shared", f"-I{headers}", str(CSRC / "pycall.c"), "-o", str(tmp)]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode == 0:
-        os.replace(tmp, out)
-    elif verbose:
-        sys.stderr.write(proc.stderr)
+    compiler the library is called through ctypes instead, which is slower, hence the warning."""
+    out = _call_module_path()
+    compiler = _call_compiler()
+    reason = "no C compiler or no Python headers"
+    if compiler is not None:
+        tmp = out.with_suffix(".tmp")
+        cmd = [*compiler, "-O2", "-Wall", "-fPIC", "-shared", str(CSRC / "pycall.c"), "-o", str(tmp)]
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if proc.returncode == 0:
+            os.replace(tmp, out)
+            return
+        reason = proc.stderr
+    out.unlink(missing_ok=True)  # not one of another version
+    warnings.warn(f"chord_b200._call was not built, calls go through ctypes (some 4 us each): {reason}")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -81,7 +102,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     obj_dir.mkdir(exist_ok=True)
     with concurrent.futures.ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
         objs = list(pool.map(lambda s: _compile(nvcc, s, obj_dir, verbose), SOURCES))
-    _build_call_module(verbose)
+    _build_call_module()
     tmp = LIB_PATH.with_suffix(".so.tmp")
     cmd = [nvcc, *ARCH_FLAGS, "-shared", "-o", str(tmp), *map(str, objs)]
     proc = subprocess.run(cmd, capture_output=True, text=True)

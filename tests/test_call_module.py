@@ -17,12 +17,52 @@ def test_native_calls_agree_with_ctypes(native_lib):
         _lib.check(native.chord_b200_indexed(*arguments))
 
 
+needs_module = pytest.mark.skipif(_lib._call is None, reason="the call module was not built")
+
+
+@needs_module
 def test_arguments_that_are_no_integers(native_lib):
-    if _lib._call is None:
-        pytest.skip("the call module was not built")
     with pytest.raises(TypeError):
         _lib.native().chord_b200_masked_tile_m("8")
+    with pytest.raises(TypeError):
+        _lib.native().chord_b200_masked_tile_m(None)
+    with pytest.raises(TypeError):
+        _lib.native().chord_b200_masked_tile_m(8.0)
     with pytest.raises(OverflowError):
         _lib.native().chord_b200_masked_tile_m(1 << 70)
-    with pytest.raises(TypeError, match="at most 24"):
-        _lib.native().chord_b200_masked_tile_m(*range(25))
+
+
+@needs_module
+@pytest.mark.parametrize("count", [0, 2, 3, 5, 25])
+def test_wrong_numbers_of_arguments(native_lib, count):
+    with pytest.raises(TypeError, match=f"takes 4 arguments.*got {count}"):
+        _lib.native().chord_b200_indexed_block_m(*range(count))
+
+
+def test_none_is_the_null_pointer(native_lib):
+    for lib in (_lib.native(), native_lib):
+        assert lib.chord_b200_silu_mul(None, 1 << 40, 4, 64, None) == 1
+        assert "null tensor pointer" in _lib.last_error()
+
+
+def test_module_counts_as_part_of_the_build(native_lib, monkeypatch, tmp_path):
+    from chord_b200 import build
+
+    assert build.is_fresh()
+    monkeypatch.setattr(build, "_call_module_path", lambda: tmp_path / "_call.so")
+    if build._call_compiler() is not None:
+        assert not build.is_fresh()
+    monkeypatch.setattr(build, "_call_compiler", lambda: None)
+    assert build.is_fresh()
+
+
+def test_failed_module_build_is_reported(native_lib, monkeypatch, tmp_path):
+    from chord_b200 import build
+
+    stale = tmp_path / "_call.so"
+    stale.write_bytes(b"of an earlier version")
+    monkeypatch.setattr(build, "_call_module_path", lambda: stale)
+    monkeypatch.setattr(build, "_call_compiler", lambda: ["false"])
+    with pytest.warns(UserWarning, match="ctypes"):
+        build._build_call_module()
+    assert not stale.exists()
