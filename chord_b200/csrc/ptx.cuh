@@ -213,6 +213,12 @@ __device__ __forceinline__ void mbar_wait_sticky(uint32_t bar, uint32_t parity, 
       : "memory");
 }
 
+// For the way out of a kernel that has given up: waits (bounded as well, about 16 ms) for a phase
+// that copies already issued will complete.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  for (int tries = 0; tries < 4096 && !mbar_try_wait<false>(bar, parity); ++tries) {}
+}
+
 // --------------------------------------------------------------------- TMA --
 
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap) {

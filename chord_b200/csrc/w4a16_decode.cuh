@@ -253,7 +253,10 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
         for (int i = 0; i < 4; ++i) acc[b][m][n][i] = 0.0f;
 
   // The waits record a failure in `bad` and the code runs on (on stale data, within this
-  // worker's own shared memory); `bad` is tested once per stage.
+  // worker's own shared memory); `bad` is tested once per stage.  It is the same in all lanes:
+  // a converged warp makes each try, each look at the abort flag and each reading of the clock
+  // as one instruction.
+  __syncwarp();
   if (ring.bad == 0) {
     for (int32_t kb = seg.kb; kb < seg.ke; ++kb) {
       const uint32_t st = ring.base + ring.off;
@@ -478,7 +481,6 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     StepStream steps;
     steps.init(tiles, k_steps, workers, worker_id);
     StageCursor cur;
-    uint32_t issued = 0;  // stages handed to the TMA so far, up to the ring's depth
     uint32_t bad = 0;
     int32_t w_row = 0, s_row = 0, w_col = 0;
     int32_t x_off[kRounds];
@@ -526,24 +528,14 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         }
       }
       ptx::cp_async_arrive_noinc(full);
-      if (issued < stages) ++issued;
       cur.advance(stages);
     }
-    // Nothing may stay in flight towards shared memory when the CTA retires: the gathers
-    // are waited for here, the TMA boxes by the computing warps, unless those gave up; then
-    // this warp waits for the stages it issued last (bounded as well).
+    // Nothing may stay in flight towards shared memory when the CTA retires, also when the
+    // computing warps give up after this warp has issued its last stage: the gathers and the
+    // boxes are waited for here (bounded), whoever else waits for them.
     ptx::cp_async_wait_all();
-    if (bad != 0) {
-      for (uint32_t i = 0; i < issued; ++i) {
-        if (cur.s == 0) {
-          cur.s = stages;
-          cur.ph ^= 1u;
-        }
-        --cur.s;
-        for (int tries = 0; tries < 4096 && !ptx::mbar_try_wait<false>(full0 + cur.s * 8u, cur.ph); ++tries) {}
-      }
-      if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
-    }
+    for (uint32_t s = 0; s < stages; ++s) ptx::mbar_drain(full0 + s * 8u, cur.last_phase(s));
+    if (bad != 0 && lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
     __syncwarp();
   } else {
     // ---------------------------------------------------------- computing warps --

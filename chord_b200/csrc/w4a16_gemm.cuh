@@ -64,6 +64,7 @@
 #include <cuda.h>
 
 #include "ptx.cuh"
+#include "ring.h"
 
 namespace chord {
 
@@ -381,26 +382,6 @@ __device__ __forceinline__ void dequant_fragment(uint32_t w, uint32_t scales, ui
       : "=&r"(d0), "=&r"(d1), "=&r"(d2), "=&r"(d3)
       : "r"(w), "r"(scales), "r"(0x43084308u));
 }
-
-// Ring position advanced without divisions (a lone issuing thread pays ~100
-// cycles for an integer division by a runtime value).
-struct StageCursor {
-  uint32_t s = 0, ph = 0;
-  __device__ __forceinline__ void advance(uint32_t stages) {
-    if (++s == stages) {
-      s = 0;
-      ph ^= 1u;
-    }
-  }
-  // Any distance, without a division (a few subtractions per tile at most).
-  __device__ __forceinline__ void advance_by(uint32_t n, uint32_t stages) {
-    s += n;
-    while (s >= stages) {
-      s -= stages;
-      ph ^= 1u;
-    }
-  }
-};
 
 // Activation ring cut into sub-slots of 128 token rows (both 64-wide K halves, 32 KB).
 // A stage of a tile of at most 128 tokens takes one sub-slot, a 256-token stage an
