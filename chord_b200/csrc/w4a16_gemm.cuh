@@ -257,6 +257,7 @@ struct __align__(16) GemmShared {
   uint64_t aempty[2 * kMaxAStages];  // per K half: its MMAs have completed (1 commit)
   uint64_t dfull[2];
   uint64_t dempty[2];
+  uint64_t mma_done;             // all MMAs issued have completed (one commit per issuer, at the end)
   uint32_t tmem_base;
   uint32_t abort_flag;
   int32_t m_blocks;
@@ -408,6 +409,12 @@ struct XSubRing {
   __device__ __forceinline__ void flip(uint32_t slot) { phases ^= 1u << slot; }
 };
 
+// Waits (bounded) for the latest use of every stage of a ring: nothing may stay in flight towards
+// shared memory when a CTA retires, also when whoever reads the stages has given up.
+__device__ __forceinline__ void drain_ring(const uint64_t* full, const StageCursor& issued, uint32_t stages) {
+  for (uint32_t i = 0; i < stages; ++i) ptx::mbar_drain(ptx::smem_u32(full + i), issued.last_phase(i));
+}
+
 template <int kDequantGroups, bool kPair>
 __global__ void __launch_bounds__(32 * (12 + 4 * kDequantGroups), 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s,
@@ -506,6 +513,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       ptx::mbar_init(ptx::smem_u32(&sh.dfull[d]), ni);
       ptx::mbar_init(ptx::smem_u32(&sh.dempty[d]), (tiled_roles ? 8u : 4u) << p.pair);
     }
+    ptx::mbar_init(ptx::smem_u32(&sh.mma_done), ni);
     sh.abort_flag = 0;
     sh.epilogue_failed = 0;
     ptx::fence_barrier_init();
@@ -669,6 +677,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         sh.abort_flag = 1;
         if (p.status) atomicOr(p.status, kStatusProducerTimeout);
       }
+      if constexpr (!kPair) drain_ring(sh.wfull, cur, w_stages);
     }
     __syncwarp();
   } else if (!tiled_roles && (warp == 0 || warp == 1)) {
@@ -708,6 +717,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         sh.abort_flag = 1;
         if (p.status) atomicOr(p.status, kStatusProducerTimeout);
       }
+      if constexpr (!kPair) drain_ring(sh.wfull, cur, w_stages);
     }
     __syncwarp();
   } else if (warp == 2 || (warp == 3 && !tiled_roles)) {
@@ -783,6 +793,13 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           cur.advance(x_stages);
         }
       }
+      if (!kPair && threadIdx.x == 64) {
+        if (subslots) {
+          for (uint32_t i = 0; i < 2u * x_stages; ++i) ptx::mbar_drain(ptx::smem_u32(&sh.xfull[i]), xring.phase(i) ^ 1u);
+        } else {
+          drain_ring(sh.xfull, cur, x_stages);
+        }
+      }
     } else if (p.x_load == kXLoadGather4) {
       // Routed rows by TMA: four rows per instruction, lanes of warp 2 own the row
       // groups lane and lane + 32.
@@ -825,6 +842,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           cur.advance(x_stages);
         }
       }
+      if (warp == 2) drain_ring(sh.xfull, cur, x_stages);
     } else {
       // Routed rows by cp.async: thread = (16-byte chunk of the 256-byte stage row,
       // row modulo 4).
@@ -1102,6 +1120,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         ++segc;
       }
       if (__any_sync(0xffffffffu, bad != 0) && lane == 0 && p.status) atomicOr(p.status, kStatusMmaTimeout);
+      // Also when a role has given up, no MMA may run on into the release of tensor memory.
+      if constexpr (!kPair) {
+        if (ptx::elect_one()) ptx::mma_commit(ptx::smem_u32(&sh.mma_done));
+        __syncwarp();
+        ptx::mbar_drain(ptx::smem_u32(&sh.mma_done), 0);
+      }
     }
     __syncwarp();
   } else if (warp >= kFirstDequantWarp && warp < kFirstEpilogueWarp) {
@@ -1469,8 +1493,17 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   ptx::tc_fence_before();
   __syncthreads();
   // `pair`: neither CTA may leave (or free tensor memory) while the other can still
-  // signal its barriers or have MMAs reading its shared and tensor memory.
-  if constexpr (kPair) ptx::cluster_sync();
+  // signal its barriers or have MMAs reading its shared and tensor memory.  After a failure
+  // boxes and MMAs of either may be under way that nobody waits for; a barrier of this CTA does
+  // not tell about the other's, so they are left a millisecond, a thousand times what they
+  // take.  (Waiting for them by role, as the other instantiation does, made every launch of
+  // this one 2 % slower.)
+  if constexpr (kPair) {
+    if (sh.abort_flag != 0) {
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
+    ptx::cluster_sync();
+  }
   if (warp == 2) {
     ptx::tc_fence_after();
     if constexpr (kPair) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
