@@ -253,14 +253,14 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
         for (int i = 0; i < 4; ++i) acc[b][m][n][i] = 0.0f;
 
   // The waits record a failure in `bad` and the code runs on (on stale data, within this
-  // worker's own shared memory); `bad` is tested once per stage.  It is the same in all lanes:
-  // a converged warp makes each try, each look at the abort flag and each reading of the clock
-  // as one instruction.
+  // worker's own shared memory); `bad` is tested once per stage.  It is the same in all lanes
+  // (the lanes vote inside the wait), so that a failure never splits the warp around the matrix
+  // instructions and the barriers below.
   __syncwarp();
   if (ring.bad == 0) {
     for (int32_t kb = seg.kb; kb < seg.ke; ++kb) {
       const uint32_t st = ring.base + ring.off;
-      ptx::mbar_wait_sticky(ring.full0 + ring.bar, ring.ph, ring.abort_addr, ring.bad);
+      ptx::mbar_wait_sticky<true>(ring.full0 + ring.bar, ring.ph, ring.abort_addr, ring.bad);
       // (the last stage holds one K half only when K is an odd multiple of 64)
       const bool second = !(tail && kb == seg.ke - 1);
       if (kBlocks == 1 || (kb & 1) == 0) {
