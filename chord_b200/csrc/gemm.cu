@@ -131,9 +131,9 @@ int resident_pairs(size_t smem) {
     config.attrs = attribute;
     config.numAttrs = 1;
     int clusters = 0;
-    cudaFuncSetAttribute(w4a16_gemm_kernel<kGroups, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(w4a16_gemm_kernel<kGroups, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(smem));
-    if (cudaOccupancyMaxActiveClusters(&clusters, w4a16_gemm_kernel<kGroups, true>, &config) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, w4a16_gemm_kernel<kGroups, true, true>, &config) != cudaSuccess) {
       cudaGetLastError();
       clusters = 0;
     }
@@ -166,7 +166,10 @@ int pick_w_stages(const DeviceInfo& dev, int mma_n, int x_stages) {
 
 template <int kGroups>
 int launch_with_groups(const CUtensorMap& tm_w, const CUtensorMap& tm_s, const CUtensorMap& tm_x,
-                       const GemmParams& p, int grid, size_t smem, cudaStream_t stream) {
+                       const GemmParams& p, bool hold, int grid, size_t smem, cudaStream_t stream) {
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
+  static const Kernel kernels[3] = {w4a16_gemm_kernel<kGroups, false, false>, w4a16_gemm_kernel<kGroups, false, true>,
+                                    w4a16_gemm_kernel<kGroups, true, true>};
   static std::once_flag flags[64];
   static cudaError_t attr_result[64];
   int device = 0;
@@ -175,11 +178,9 @@ int launch_with_groups(const CUtensorMap& tm_w, const CUtensorMap& tm_s, const C
     DeviceInfo dev;
     int max_optin = 227 * 1024;
     if (current_device_info(&dev) == kOk) max_optin = dev.max_smem_optin;
-    attr_result[device & 63] = cudaFuncSetAttribute(
-        w4a16_gemm_kernel<kGroups, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin);
-    if (attr_result[device & 63] == cudaSuccess) {
-      attr_result[device & 63] = cudaFuncSetAttribute(
-          w4a16_gemm_kernel<kGroups, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin);
+    for (const Kernel kernel : kernels) {
+      const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin);
+      if (attr_result[device & 63] == cudaSuccess) attr_result[device & 63] = rc;
     }
   });
   if (attr_result[device & 63] != cudaSuccess) {
@@ -187,14 +188,13 @@ int launch_with_groups(const CUtensorMap& tm_w, const CUtensorMap& tm_s, const C
                 cudaGetErrorString(attr_result[device & 63]));
   }
   const int threads = 32 * (12 + 4 * kGroups);
+  const Kernel kernel = kernels[p.pair ? 2 : (hold ? 1 : 0)];
   if (p.pair) {
     // every CTA has to be resident (stream-K owners wait for their contributors)
-    CHORD_CUDA(launch_kernel_pairs(w4a16_gemm_kernel<kGroups, true>, dim3(grid), dim3(threads), smem, stream,
-                                   p.pdl != 0, tm_w, tm_s, tm_x, p));
+    CHORD_CUDA(launch_kernel_pairs(kernel, dim3(grid), dim3(threads), smem, stream, p.pdl != 0, tm_w, tm_s, tm_x, p));
     return kOk;
   }
-  CHORD_CUDA(launch_kernel(w4a16_gemm_kernel<kGroups, false>, dim3(grid), dim3(threads), smem, stream,
-                           p.pdl != 0, tm_w, tm_s, tm_x, p));
+  CHORD_CUDA(launch_kernel(kernel, dim3(grid), dim3(threads), smem, stream, p.pdl != 0, tm_w, tm_s, tm_x, p));
   return kOk;
 }
 
@@ -510,8 +510,15 @@ int launch_gemm(GemmParams p, const void* x, const int32_t* packed, const void* 
                       static_cast<size_t>(p.w_stages) * (kWStageBytes + kSStageBytes) +
                       fixed_smem_bytes();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (options().dequant_groups == 4) return launch_with_groups<4>(tm_w, tm_s, tm_x, p, launch_grid, smem, s);
-  return launch_with_groups<2>(tm_w, tm_s, tm_x, p, launch_grid, smem, s);
+  // Accumulators of more than 128 columns in all are single-buffered: those are read into registers
+  // and handed back before a tile's rows are stored (kHold, an instantiation of its own: within
+  // the general one the 64 registers spill, and every launch paid for that, us, before / as
+  // part of the general one / now: 24 experts of 1536 x 4096, contiguous, 256 rows each 100.7 /
+  // 106.9 / 97.6, 85 rows 75.0 / 75.3 / 67.8; 32 of 2048 x 2048, fused, 110 rows 70.4 / 76.1 / 69.4; 48 of
+  // 7168 x 2048, 85 rows 196 / 177 / 169).
+  const bool hold = p.pair || (p.npair && !p.fuse_silu && p.mma_n > 64);
+  if (options().dequant_groups == 4) return launch_with_groups<4>(tm_w, tm_s, tm_x, p, hold, launch_grid, smem, s);
+  return launch_with_groups<2>(tm_w, tm_s, tm_x, p, hold, launch_grid, smem, s);
 }
 
 // Stream-K scratch that lives in the library image instead of in an allocation:

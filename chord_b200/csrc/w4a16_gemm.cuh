@@ -415,7 +415,10 @@ __device__ __forceinline__ void drain_ring(const uint64_t* full, const StageCurs
   for (uint32_t i = 0; i < stages; ++i) ptx::mbar_drain(ptx::smem_u32(full + i), issued.last_phase(i));
 }
 
-template <int kDequantGroups, bool kPair>
+// kPair: clusters of two CTAs (p.pair).  kHold: two weight blocks per tile (on one CTA or on a
+// pair), without SiLU*mul; whole tiles are held in registers while they are stored (see the
+// epilogue).
+template <int kDequantGroups, bool kPair, bool kHold>
 __global__ void __launch_bounds__(32 * (12 + 4 * kDequantGroups), 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s,
                   const __grid_constant__ CUtensorMap tm_x, const GemmParams p) {
@@ -466,7 +469,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   // of two partial sums.  An activation tile then crosses from L2 to the SM once per 256
   // weight rows instead of once per 128: with 128-row tiles the kernel was bound by that
   // traffic (about 10 TB/s between L2 and the SMs), not by the tensor pipe.
-  const bool npair = p.npair != 0;
+  static_assert(kHold || !kPair, "tiles on CTA pairs are always held");
+  const bool npair = !kPair && (kHold || p.npair != 0);
   const int32_t w_per_kb = npair ? 2 : 1;  // weight/scale ring entries per K block
   // 256-token layouts with consecutive activation rows: sub-slot ring (see XSubRing).
   const bool subslots = ksplit && p.x_load == kXLoadTiled && p.mma_n == 256;
@@ -484,7 +488,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   // taking every other 16-column chunk.  Accumulators of 128 columns and more are
   // single-buffered, so the tensor core idles while a tile is drained: with K = 2048 the
   // four-warp drain was a quarter of the time of a two-block tile.
-  const bool tiled_roles = kPair || (p.x_load == kXLoadTiled && ni <= 2u);
+  const bool tiled_roles = kHold || (p.x_load == kXLoadTiled && ni <= 2u);
   const uint32_t epi_threads = tiled_roles ? 256u : 128u;
 
   // ------------------------------------------------------------------ setup --
@@ -1303,7 +1307,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       const uint32_t seg_len = static_cast<uint32_t>(seg.ke - seg.kb);
       // Fused SiLU*mul: one pass, which reads both accumulators (gate, up), combines them
       // and writes a [rows, N/2] tensor.
-      const bool fuse = p.fuse_silu != 0;
+      const bool fuse = !kHold && p.fuse_silu != 0;
       const int32_t ldn = fuse ? (p.n >> 1) : p.n;
       __nv_bfloat16* stage = &sh.stage[egroup * 4u + q][0][0];
       // Transpose of 16 tokens through shared memory so that global stores are 16 bytes wide:
@@ -1330,15 +1334,15 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         }
         __syncwarp();
       };
-      if ((kPair || npair) && seg.type == kSegFull) {
-        // A whole tile on eight epilogue warps: the warp's share of the accumulators (at most
-        // eight chunks of 16 columns) is read and rounded first, the accumulators go back to
-        // the issuers, and only then are the rows written.  Accumulators of this size are
-        // single-buffered: what is left between two tiles is the reading alone.
+      if (kHold && seg.type == kSegFull) {
+        // The warp's share of the accumulators (at most eight chunks of 16 columns) is read and
+        // rounded first, the accumulators go back to the issuers, and only then are the rows
+        // written.  Accumulators of this size are single-buffered: what is left between two
+        // tiles is the reading alone.
         constexpr int kChunks = 8;
         uint32_t held[kChunks][8];
         const int32_t first = static_cast<int32_t>(egroup) * 16;
-        const bool two_blocks = !kPair && !fuse;  // chunks 4-7 are the second weight block's
+        constexpr bool two_blocks = !kPair;  // chunks 4-7 are the second weight block's
 #pragma unroll
         for (int i = 0; i < kChunks; ++i) {
           const int32_t c0 = first + 32 * (two_blocks ? (i & 3) : i);
@@ -1350,19 +1354,6 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           uint32_t v[16];
           ptx::tmem_ld_32x32b_x16(d_addr + (two_blocks ? (i >> 2) * d_cols : 0u) + c0, v);
           ptx::tmem_wait_ld();
-          if (fuse) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t u[8];
-              ptx::tmem_ld_32x32b_x8(d_addr + d_cols + c0 + 8 * h, u);
-              ptx::tmem_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const float gate = __uint_as_float(v[8 * h + j]);
-                v[8 * h + j] = __float_as_uint(gate / (1.0f + __expf(-gate)) * __uint_as_float(u[j]));
-              }
-            }
-          }
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const __nv_bfloat162 pair2 = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
