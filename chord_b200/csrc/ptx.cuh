@@ -17,12 +17,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ uint32_t lane_id() {
-  uint32_t v;
-  asm volatile("mov.u32 %0, %%laneid;" : "=r"(v));
-  return v;
-}
-
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -275,16 +269,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       : "memory");
 }
 
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const void* tmap, uint32_t bar,
-                                                 int32_t c0, int32_t c1, uint64_t hint) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%3, %4}], [%2], %5;"
-      :
-      : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "l"(hint)
-      : "memory");
-}
-
 // Four rows (r0..r3) of a 2-D tensor, columns [c0, c0 + box width), land as
 // four consecutive box rows at dst.  Rows outside the tensor read as zero.
 __device__ __forceinline__ void tma_gather4(uint32_t dst, const void* tmap, uint32_t bar,
@@ -298,10 +282,6 @@ __device__ __forceinline__ void tma_gather4(uint32_t dst, const void* tmap, uint
         "r"(r2), "r"(r3)
       : "memory");
 }
-
-// L2 eviction-priority descriptors for the .L2::cache_hint TMA forms.
-constexpr uint64_t kEvictFirst = 0x12F0000000000000ull;
-constexpr uint64_t kEvictLast = 0x14F0000000000000ull;
 
 // 8-byte shared-memory load from a 32-bit shared address plus a compile-time offset
 // (the offset folds into the instruction, so unrolled loads share one address register).
@@ -417,20 +397,6 @@ __device__ __forceinline__ void mma_ts_k64(uint32_t d_tmem, uint32_t a_tmem, uin
       : "memory");
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc].
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // Arrives (count 1) on `bar` once every tcgen05.mma issued so far by this
 // thread has completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -460,16 +426,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32"
-      " {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(taddr)
-      : "memory");
-}
-
 // 16 lanes x 32 columns.  Thread t of the warp supplies, for column group u
 // (columns 4u .. 4u+3): r[2u] -> (lane t/4, column 4u + t%4) and
 // r[2u+1] -> (lane t/4 + 8, column 4u + t%4).
@@ -481,17 +437,6 @@ __device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_
       : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
         "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
         "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
-// 32 lanes x 8 columns: thread i writes lane (base + i), register j to column j.
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32"
-      " [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-      :
-      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-        "r"(r[7])
       : "memory");
 }
 
@@ -635,14 +580,6 @@ __device__ __forceinline__ int ld_acquire(const int* addr) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
-}
-
-// Shared-memory counter increment that orders the caller's earlier writes before it
-// and later reads after it (CTA scope); returns the previous value.
-__device__ __forceinline__ uint32_t atom_add_acq_rel_shared(uint32_t addr, uint32_t v) {
-  uint32_t old;
-  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
-  return old;
 }
 
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
