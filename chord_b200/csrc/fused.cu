@@ -143,7 +143,7 @@ int chord_b200_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int6
   CHORD_REQUIRE(expert_cap >= need / block_m, "expert_ids capacity %lld is below the worst case %lld",
                 static_cast<long long>(expert_cap), static_cast<long long>(need / block_m));
   // From 4096 ids on 32 warps, sixteen rounds of loads ahead, where the counters fit 160 KB (up
-  // to 1240 experts).  Below that the short loop of 16 warps: a batch's unrolled code costs a
+  // to 1241 experts).  Below that the short loop of 16 warps: a batch's unrolled code costs a
   // small call more (instruction fetches) than the loads it overlaps.
   // (32768 ids over 48 experts: 39.6 us with a load per round and 16 warps, 18.5 us now; 2048 ids:
   // 5.0 us with the short loop, 5.8 with the long one.)
