@@ -236,11 +236,14 @@ int64_t stream_k_bytes(int grid, int mma_n) {
   return (general + 1023) / 1024 * 1024;
 }
 
-// CTA pairs pay off on tiles of more than 128 tokens: a pair MMA costs its issuing thread
-// about 130 cycles whatever its N (measured at 85 and 128 rows per expert: 490 / 505 us on
-// pairs against 388 / 419 us on the two-issuer layout; at 256 and 512 rows: 591 / 1131 us
-// against 720 / 1386 us).  The single 256-column accumulator is drained between tiles with
-// the tensor core idle, so very short K loops are left to single CTAs.
+// CTA pairs pay off on tiles of more than 128 tokens, where each CTA loads half of the rows (48
+// experts of 4096 x 7168, us: 256 / 512 rows each 591 / 1131 against 720 / 1386 on single
+// CTAs).  Tiles of at most 128 tokens are faster as two blocks on one CTA with an issuer for
+// each: 48 experts of 4096 x 7168, 85 / 128 rows each 354 / 404 against 389 / 435 us, of 7168
+// x 2048 167 / 194 against 194 / 211; few and short tiles are not (32 experts of 2048 x 2048, 100
+// rows: 63 against 55).  The line in K was drawn when a tile was stored before its accumulator
+// went back to the issuer; now that it is held in registers, shorter K would gain from pairs
+// too (16 experts of 3072 x 1024, 250 rows: 58 us on single CTAs, 47 on pairs).
 bool pair_applies(int mma_n, int n, int k) {
   return options().pair != 0 && mma_n > 128 && k >= 2048 && (n / kBlockN) % 2 == 0;
 }
@@ -255,8 +258,8 @@ bool pairs_resident(const DeviceInfo& dev) {
 bool pregather_applies(int mma_n) { return options().pregather != 0 && mma_n >= 64; }
 
 // Token tiles of at most 32 rows (indexed, masked) have a kernel of their own, in which
-// every warpgroup of a CTA is an independent worker with a lock word and a scratch
-// slot of its own: four times as many of each as the general kernel needs.
+// a CTA is four independent workers, each with a lock word and a scratch slot of its
+// own: four times as many of each as the general kernel needs.
 bool decode_kernel_applies(const GemmParams& p) {
   return options().decode_kernel != 0 && p.mode != kModeContiguous && p.mma_n <= kDecMaxTokens;
 }
@@ -351,7 +354,7 @@ int launch_gemm(GemmParams p, const void* x, const int32_t* packed, const void* 
   p.lock_spins = options().lock_spins;
   if (options().pdl != 0) p.pdl = 1;
   // The decode kernel runs when the caller's locks and scratch are large enough for
-  // one per warpgroup; with the smaller buffers of the general kernel, that one runs.
+  // one per worker; with the smaller buffers of the general kernel, that one runs.
   // SiLU*mul fused into the gate_up epilogue: on the decode kernel for 16-token tiles (two
   // accumulators of 16 columns: twice the scratch slot), on the general kernel for tiles that
   // span a gate and an up block (`npair` layout).
@@ -562,6 +565,12 @@ int chord_b200_indexed_block_m(int64_t n, int64_t k, int64_t num_experts, int64_
   // Rows per local expert if the routes spread evenly; the tile's token
   // dimension is the MMA N, whose minimum is 16, so smaller blocks buy nothing.
   const double avg = static_cast<double>(routed_m) / static_cast<double>(num_experts);
+  // Poisson counts, us with the smaller / the larger block around each line (weights from HBM):
+  //   line   average   48 of 4096 x 7168   48 of 7168 x 2048   64 of 1024 x 1024
+  //   8      8, 14     174/191 246/250     97/109 122/132      16/17 24/21
+  //   20     18, 24    294/261 309/265     145/150 154/146     22/32 22/34
+  //   44     40, 64    299/309 404/344     164/158 221/167     36/35 46/38
+  //   100    100, 140  378/412 578/509     187/229 304/257     42/54 46/64
   if (avg <= 8.0) return 16;
   if (avg <= 20.0) return 32;
   if (avg <= 44.0) return 64;
@@ -571,7 +580,12 @@ int chord_b200_indexed_block_m(int64_t n, int64_t k, int64_t num_experts, int64_
 
 int chord_b200_masked_tile_m(int64_t expected_m) {
   // A group with more rows than the tile costs a second pass over its weights, so the
-  // tile leaves room for the spread around the expected count.
+  // tile leaves room for the spread around the expected count.  24 groups, Poisson counts,
+  // us with the smaller / the larger tile around each line:
+  //   line   expected   4096 x 7168   7168 x 2048   512 x 2048
+  //   8      8, 12      96/110 117/125   53/59 61/69   15/16 15/18
+  //   20     16, 20     144/131 151/136  77/78 85/78   19/20 19/20
+  //   48     44, 56     154/147 173/160  90/83 102/82  22/21 22/22
   if (expected_m <= 8) return 16;
   if (expected_m <= 20) return 32;
   if (expected_m <= 48) return 64;
@@ -581,14 +595,15 @@ int chord_b200_masked_tile_m(int64_t expected_m) {
 
 // From an expected 121 rows on many groups exceed a 128-row tile and would pay a second pass
 // over their weights: 256-row tiles instead, where those run on CTA pairs.  128- against 256-row
-// tiles, us, weights from HBM:
+// tiles, us, weights from HBM (the Poisson counts are one draw each; that at 128 has few groups
+// above 128):
 //   24 groups, Poisson counts      4096 x 7168   7168 x 2048   512 x 2048
-//     112 expected                 181 / 209     119 / 106     29 / 26
-//     121                          218 / 199     124 / 106     28 / 27
-//     128                          281 / 200     156 / 112     33 / 28
-//     144                          285 / 212     173 / 116     37 / 29
-//   128 rows in every group        174 / 193     117 / 109     28 / 26
-//     16 (expected_m far too high) 132 / 157     86 / 95       20 / 19
+//     112 expected                 170 / 221     96 / 113      26 / 25
+//     121                          224 / 207     127 / 114     26 / 26
+//     128                          203 / 213     117 / 116     26 / 26
+//     144                          300 / 239     170 / 120     31 / 28
+//   128 rows in every group        193 / 203     116 / 122     26 / 25
+//     16 (expected_m far too high) 146 / 159     94 / 95       18 / 18
 int chord_b200_masked_tile_rows(int64_t expected_m, int64_t max_m, int64_t n, int64_t k) {
   chord::OptionsReadLock options_guard(chord::options_mutex());
   const int tile_m = chord_b200_masked_tile_m(expected_m);

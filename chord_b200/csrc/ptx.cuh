@@ -87,10 +87,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 // warp until it completes or an implementation-defined limit (measured: ~4 us) runs out.
 // Parked warps take no issue slots, which matters here: most warps of a CTA wait on
 // barriers much of the time, and a hot spin would crowd out the ones that work.
-// Two forms.  With a suspend-time hint the compiler emits try, nanosleep, try: the
-// general kernel, whose waiters are mostly lone threads, measured 3-7 % faster with it.
-// Without a hint it is a single instruction: the decode kernel, whose 24 warps all
-// wait warp-wide, measured 2.5 % faster with that.
+// Two forms.  With a suspend-time hint the compiler emits try, nanosleep, try: for the
+// general kernel's producers and epilogue.  Without a hint it is a single instruction: for
+// warps on the path from a stage to its product (mbar_wait_sticky below), which wait often
+// and briefly.
 constexpr uint32_t kSuspendHintNs = 200000;
 
 template <bool kHint = true>
@@ -158,10 +158,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
 // try as one instruction on one address, so its first outcome is the same in every
 // lane; only the slow path can end differently per lane, and there the warp votes so
 // that a timeout never splits it.
-template <bool kHint = true>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile uint32_t* abort_flag) {
-  if (mbar_try_wait<kHint>(bar, parity)) return true;
+  if (mbar_try_wait(bar, parity)) return true;
   const bool ok = mbar_wait_slow(bar, parity, abort_flag);
   return __all_sync(__activemask(), ok);
 }

@@ -24,28 +24,32 @@
 // deep enough (20+ stages of 9 KB) to cover HBM latency, while an activation
 // stage stays until the MMAs that read it have completed.
 //
-// The single-thread issue loops (TMA, MMA) are kept free of divisions and
-// descriptor rebuilds: one lone thread retires a dependent instruction only
-// every few cycles, and at decode sizes a K16 MMA has roughly 45 cycles of HBM
-// time to hide behind.
+// The issue loops (TMA: one thread, MMA: a warp with an elected lane) are kept free of
+// divisions and descriptor rebuilds: each is one chain of dependent instructions, of which
+// a warp retires one only every few cycles, and at decode sizes a K16 MMA has roughly 45
+// cycles of HBM time to hide behind.
 //
 // Warp roles (one CTA per SM, persistent):
 //   warp 0            producer: TMA for packed weights
 //   warp 1            producer: TMA for scales
 //   warps 2-3         activations: tiled TMA (one thread), cp.async gather (64 threads)
 //                     or TMA gather4 (one warp); warp 2 also allocates tensor memory
-//   warps 4-7         MMA issuers, one thread each; issuer i takes the stages
-//                     with index = i modulo the issuer count and owns one accumulator
+//   warps 4-7         MMA issuers; issuer i takes the stages with index = i modulo the
+//                     issuer count and owns one accumulator
 //   warps 8..8+4G-1   G dequant groups of four warps (one per TMEM lane quarter)
 //   last four warps   epilogue: TMEM -> registers -> BF16 -> global, plus the
 //                     stream-K reduction through `locks` and the FP32 workspace
+// Where the activation rows are consecutive and at most two issuers run (`tiled_roles`), warp 0
+// loads weights and scales, warps 1 and 3 issue, and warps 4-7 are a second group of
+// epilogue warps.
 //
-// Why several issuers: one thread can issue a tcgen05.mma only every ~56 cycles
-// (measured), while a 128x16 tile of packed weights arrives from HBM every ~45
-// cycles per SM.  With small token tiles (decode) the stages are therefore
+// Why several issuers: an issuer's chain per K16 (its share of the waits, an MMA, its share of
+// the commits) is longer than the ~45 cycles in which a 128x16 tile of packed weights
+// arrives from HBM per SM.  With small token tiles (decode) the stages are therefore
 // dealt to 2 or 4 issuers in different warps, each accumulating into its own
 // TMEM columns; the epilogue adds the accumulators in issuer order, so the
-// result does not depend on timing.  Large token tiles use a single issuer.
+// result does not depend on timing.  Large token tiles use a single issuer, tiles of two
+// weight blocks one per block.
 //
 // Scheduling follows the reference's scheme (humming/scheduler.cuh:73-101):
 // whole tiles are dealt round-robin to the CTAs while full waves last; the

@@ -235,7 +235,7 @@ int chord_b200_indexed_slots(const void* x, const int32_t* packed, const void* s
  *    refused with return code 1 and a message naming the limit.
  *  - Which kernel runs follows from what fits into the 5 MiB: with block_m <= 16 the
  *    decode kernel, as for chord_b200_indexed (results bit-equal to it).  With
- *    block_m 17..32 the decode kernel's one slot per warpgroup (9.7 MB on 148 SMs) does
+ *    block_m 17..32 the decode kernel's one slot per worker (9.7 MB on 148 SMs) does
  *    not fit, so the general kernel runs where chord_b200_indexed would run the decode
  *    kernel: same results within the output tolerance, not bit-equal, and slower.
  *    With block_m 33..64 there is no room for the slot-ordered copy of the routed
