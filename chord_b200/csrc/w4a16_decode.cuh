@@ -25,11 +25,13 @@
 //   * a tile runs with 8, 16 or 32 token columns, by the rows it really has: at decode
 //     sizes most routing blocks of 16 hold at most 8.
 //
-// Measured on a B200, gate_up [4096, 7168] / down [7168, 2048] of 48 local experts, top-8 of
-// 384, tcgen05 version -> this one: 1 token 19.5 / 14.7 -> 12.4 / 10.0 us (no tensor memory to
-// allocate, no activation buffer to clear), 16 tokens 36.7 / 25.5 -> 28.9 / 18.9 us, 64
-// tokens 136 / 82 -> 116 / 66 us, 256 tokens 187 / 109 -> 161 / 87 us (5.0 / 4.6 TB/s of
-// packed weights and scales).
+// Measured on a B200, gate_up [4096, 7168] / down [7168, 2048] of a layer's local experts, top-8
+// of 384, weights from HBM, replayed graph, tcgen05 version -> this one: 1 token (one expert
+// reached) 19.2 / 14.7 -> 12.8 / 10.3 us (no tensor memory to allocate, no activation buffer to
+// clear), 16 tokens (11 experts) 53.7 / 34.5 -> 44.0 / 27.8 us, 64 tokens (34) 134 / 80 -> 111 / 65 us,
+// 256 tokens (48) 188 / 111 -> 156 / 88 us (5.1 / 4.5 TB/s of packed weights and scales).
+// From 11 to 48 experts a launch takes 3.0 / 1.65 us per expert (5.5 / 5.0 TB/s) and 11 / 10 us
+// beside them: set-up, the first stages, and the stream-K slices at the end.
 #pragma once
 
 #include "w4a16_gemm.cuh"
