@@ -36,6 +36,7 @@ reference's CPU torch path (oracle/w4a16_oracle.py) on a bounded sample of the w
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
 import sys
@@ -84,11 +85,16 @@ def measured_peaks():
 
 def recorded_traffic():
     """DRAM bytes per step of the decode kernel's two launches from the committed ncu
-    capture (profiles/w4a16_decode_kernel_traffic.json), or None."""
+    capture (profiles/w4a16_decode_kernel_traffic.json), or None if there is none of the
+    kernel as it stands (the record holds the hash of the source it was captured on)."""
     path = ROOT / "profiles" / "w4a16_decode_kernel_traffic.json"
     if not path.exists():
         return None
-    return json.loads(path.read_text())
+    record = json.loads(path.read_text())
+    source = ROOT / record["source"]
+    if not source.exists() or hashlib.sha256(source.read_bytes()).hexdigest() != record["source_sha256"]:
+        return None
+    return record
 
 
 def traffic_bytes(active, n, k, in_rows, out_rows):

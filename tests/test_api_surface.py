@@ -114,3 +114,22 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setenv("CHORD_B200_LIB", str(tmp_path / "absent.so"))
     with pytest.raises(RuntimeError, match="no fallback"):
         _lib.load()
+
+
+def test_recorded_traffic_is_of_the_kernel_in_the_tree(tmp_path, monkeypatch):
+    """bench.py reports DRAM bytes of a capture only for the source the capture was taken on."""
+    import hashlib
+    import json
+
+    import bench
+
+    source = tmp_path / "kernel.cuh"
+    source.write_text("// the kernel\n")
+    record = {"source": source.name, "source_sha256": hashlib.sha256(source.read_bytes()).hexdigest(),
+              "dram_bytes_per_step": 1}
+    (tmp_path / "profiles").mkdir()
+    (tmp_path / "profiles" / "w4a16_decode_kernel_traffic.json").write_text(json.dumps(record))
+    monkeypatch.setattr(bench, "ROOT", tmp_path)
+    assert bench.recorded_traffic() == record
+    source.write_text("// another version\n")
+    assert bench.recorded_traffic() is None
