@@ -169,6 +169,58 @@ __device__ __forceinline__ void decode_x_offsets(uint32_t lane, uint32_t (&x)[4]
   }
 }
 
+// Token fragments of one K16 step (NT >= 2).
+template <int NT, int kX>
+__device__ __forceinline__ void decode_tokens(uint32_t addr, uint32_t (&b)[2 * NT]) {
+  uint32_t t[4];
+  ptx::ldmatrix_x4<kX>(addr, t);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b[i] = t[i];
+  if constexpr (NT > 2) {
+    ptx::ldmatrix_x4<kX + 2048>(addr, t);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[4 + i] = t[i];
+  }
+}
+
+// decode_half() below for any scale: a loop over the two K32 groups, small code that is hardly
+// ever run.
+template <int kTokens, int NT, int kHalf>
+__device__ __forceinline__ void decode_half_any(uint32_t st, const DecodeLane& at, float (&acc)[2][NT][4]) {
+  constexpr int kW = kTokens * 256 + 4096 * kHalf;
+  constexpr int kS = kTokens * 256 + kDecWBytes + 512 * kHalf;
+  constexpr int kX = kTokens * 128 * kHalf;
+#pragma unroll 1
+  for (uint32_t g = 0; g < 2; ++g) {
+    const uint2 scales = ptx::lds64<kS>(st + at.s + g * 256u);
+    uint2 words[2];
+    words[0] = ptx::lds64<kW>(st + at.w + g * 2048u);
+    words[1] = ptx::lds64<kW + 1024>(st + at.w + g * 2048u);
+    uint32_t b[2][2 * NT];
+    if constexpr (NT == 1) {
+      uint32_t t[4];
+      ptx::ldmatrix_x4<kX>(st + (at.x[0] ^ (g * 64u)), t);
+      b[0][0] = t[0];
+      b[0][1] = t[1];
+      b[1][0] = t[2];
+      b[1][1] = t[3];
+    } else {
+#pragma unroll
+      for (uint32_t j = 0; j < 2; ++j) decode_tokens<NT, kX>(st + (at.x[0] ^ (g * 64u + j * 32u)), b[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      uint32_t a[4];
+      dequant_fragment_any(words[j].x, scales.x, a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
+      dequant_fragment_any(words[j].y, scales.y, a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
+    }
+  }
+}
+
 // One 64-wide K half of a stage: 32 weight rows x 64 K x 8 NT tokens.
 template <int kTokens, int NT, int kHalf>
 __device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, float (&acc)[2][NT][4]) {
@@ -194,27 +246,25 @@ __device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, f
       b[2 * j + 1][1] = t[3];
     }
   }
+  if (__any_sync(0xffffffffu, scales_out_of_range(scales[0], scales[1]) != 0)) {
+    decode_half_any<kTokens, NT, kHalf>(st, at, acc);
+    return;
+  }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if constexpr (NT > 1) {
-      uint32_t t[4];
-      ptx::ldmatrix_x4<kX>(st + at.x[j], t);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) b[j][i] = t[i];
-      if constexpr (NT > 2) {
-        ptx::ldmatrix_x4<kX + 2048>(st + at.x[j], t);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) b[j][4 + i] = t[i];
-      }
-    }
+  for (int g = 0; g < 2; ++g) {
     // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
-    uint32_t a[4];
-    dequant_fragment(words[j].x, scales[j >> 1].x, a[0], a[1], a[2], a[3]);
+    const ScaleFactors fa = scale_factors(scales[g].x), fb = scale_factors(scales[g].y);
 #pragma unroll
-    for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
-    dequant_fragment(words[j].y, scales[j >> 1].y, a[0], a[1], a[2], a[3]);
+    for (int j = 2 * g; j < 2 * g + 2; ++j) {
+      if constexpr (NT > 1) decode_tokens<NT, kX>(st + at.x[j], b[j]);
+      uint32_t a[4];
+      dequant_fragment(words[j].x, fa, a[0], a[1], a[2], a[3]);
 #pragma unroll
-    for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
+      dequant_fragment(words[j].y, fb, a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
+    }
   }
 }
 
@@ -353,8 +403,8 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float v = acc[0][m][n][i];
-          if (kBlocks == 2) v = silu_f32(v) * acc[kBlocks - 1][m][n][i];
+          float v = acc[0][m][n][i] * kWeightUnit;
+          if (kBlocks == 2) v = silu_f32(v) * (acc[kBlocks - 1][m][n][i] * kWeightUnit);
           stage[(2 * c + (i & 1)) * kDecPitch + 16 * m + 8 * (i >> 1) + g] = __float2bfloat16_rn(v);
         }
       __syncwarp();
