@@ -301,6 +301,15 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
                : "memory");
 }
 
+// Two 8x8 BF16 matrices (lanes 0-15 supply the addresses).
+template <int kOffset>
+__device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2+%3];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(addr), "n"(kOffset)
+               : "memory");
+}
+
 // D[16 rows, 8 columns] += A[16, 16] * B[16, 8]: BF16 operands, FP32 accumulation, all in
 // the warp's registers.
 __device__ __forceinline__ void mma_m16n8k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

@@ -110,39 +110,6 @@ __device__ __forceinline__ TileInfo decode_tile_small(const GemmParams& p, const
   return t;
 }
 
-// The ring stages (tile, 128-wide K block) of one worker in order, one at a time.
-struct StepStream {
-  SegmentIterator iter;
-  Segment seg;
-  TileInfo t;
-  int32_t kb;
-  bool live;
-
-  __device__ void init(int32_t tiles, int32_t k_steps, int32_t workers, int32_t worker) {
-    iter.init(tiles, k_steps, workers, worker, true);
-    live = false;
-    kb = 0;
-  }
-
-  // Moves to the next step; `first` tells whether it opens a new segment.
-  __device__ bool next(const GemmParams& p, const int32_t* group_prefix, bool& first) {
-    if (live && ++kb < seg.ke) {
-      first = false;
-      return true;
-    }
-    while (iter.next(seg)) {
-      t = decode_tile_small(p, group_prefix, seg.tile);
-      if (!t.valid) continue;
-      kb = seg.kb;
-      live = true;
-      first = true;
-      return true;
-    }
-    live = false;
-    return false;
-  }
-};
-
 __device__ __forceinline__ float silu_f32(float v) { return v / (1.0f + __expf(-v)); }
 
 // Where a computing warp finds its operands: shared-memory offsets into a ring stage.
@@ -176,7 +143,12 @@ __device__ __forceinline__ void decode_tokens(uint32_t addr, uint32_t (&b)[2 * N
   ptx::ldmatrix_x4<kX>(addr, t);
 #pragma unroll
   for (int i = 0; i < 4; ++i) b[i] = t[i];
-  if constexpr (NT > 2) {
+  if constexpr (NT == 3) {
+    uint32_t u[2];
+    ptx::ldmatrix_x2<kX + 2048>(addr, u);
+    b[4] = u[0];
+    b[5] = u[1];
+  } else if constexpr (NT == 4) {
     ptx::ldmatrix_x4<kX + 2048>(addr, t);
 #pragma unroll
     for (int i = 0; i < 4; ++i) b[4 + i] = t[i];
@@ -257,13 +229,13 @@ __device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, f
 #pragma unroll
     for (int j = 2 * g; j < 2 * g + 2; ++j) {
       if constexpr (NT > 1) decode_tokens<NT, kX>(st + at.x[j], b[j]);
-      uint32_t a[4];
+      uint32_t a[4], c[4];
       dequant_fragment(words[j].x, fa, a[0], a[1], a[2], a[3]);
+      dequant_fragment(words[j].y, fb, c[0], c[1], c[2], c[3]);
 #pragma unroll
       for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
-      dequant_fragment(words[j].y, fb, a[0], a[1], a[2], a[3]);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], c, b[j][2 * n], b[j][2 * n + 1]);
     }
   }
 }
@@ -516,6 +488,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const uint32_t empty0 = ptx::smem_u32(&ws.empty[0]);
 
   if (warp < kDecWorkers) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     // ------------------------- feeder of worker `warp`: weights, scales, activations --
     // Lane 0 issues the two TMA boxes of a stage; all lanes gather its activation rows with
     // cp.async (lane l fetches the 16-byte piece l % 8 of rows l / 8 + 4 b, b < kTokens / 4,
@@ -530,57 +503,61 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const uint32_t r = r0 + 4u * b;
       dst_off[b] = r * 128u + ((piece ^ (r & 7u)) << 4);
     }
-    StepStream steps;
-    steps.init(tiles, k_steps, workers, worker_id);
+    SegmentIterator iter;
+    iter.init(tiles, k_steps, workers, worker_id, true);
+    Segment seg;
     StageCursor cur;
     uint32_t bad = 0;
-    int32_t w_row = 0, s_row = 0, w_col = 0;
-    int32_t x_off[kRounds];
-    uint32_t active = 0;  // bit b: some lane has a row to fetch in round b
-    const __nv_bfloat16* src = p.x;
-    bool first = false;
-    while (steps.next(p, sh.group_prefix, first)) {
-      const int32_t kb = steps.kb >> fuse;  // fused: both blocks read the same K block
-      if (first) {
-        active = 0;
-#pragma unroll
-        for (int b = 0; b < kRounds; ++b) {
-          const int32_t slot = static_cast<int32_t>(r0) + 4 * b;
-          int32_t off = -1;
-          if (slot < steps.t.ntok) {
-            const int32_t row = x_row_of(p, steps.t, slot);
-            if (row < p.x_rows) off = row * p.k;
-          }
-          x_off[b] = off;
-          if (__ballot_sync(0xffffffffu, off >= 0) != 0) active |= 1u << b;
-        }
-      }
-      w_row = steps.t.expert * (p.k / 16) + kb * (kDecStageK / 16);
-      s_row = steps.t.expert * (p.k / 32) + kb * (kDecStageK / 32);
-      w_col = steps.t.n0 + (fuse ? (steps.kb & 1) * (p.n >> 1) : 0);
-      src = p.x + kb * kDecStageK + piece * 8;
-      ptx::mbar_wait_sticky(empty0 + cur.s * 8u, cur.ph ^ 1u, abort_addr, bad);
-      bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
-      if (bad != 0) break;
-      const uint32_t st = ring0 + cur.s * kStageBytes;
-      const uint32_t full = full0 + cur.s * 8u;
-      if (lane == 0) {
-        ptx::mbar_arrive_expect_tx(full, kDecWSBytes);
-        ptx::tma_load_2d(st + kXBytes, &tm_w, full, 2 * w_col, w_row);
-        ptx::tma_load_2d(st + kXBytes + kDecWBytes, &tm_s, full, w_col, s_row);
-      }
-      __syncwarp();
-      const bool second_half = !(k_tail_half && steps.kb == k_steps - 1);
+    while (bad == 0 && iter.next(seg)) {
+      const TileInfo t = decode_tile_small(p, sh.group_prefix, seg.tile);
+      if (!t.valid) continue;
+      // Once per segment: where the lane's rows are; a stage then only moves the pointers on.
+      int32_t kb = seg.kb >> fuse;  // fused: both blocks of a pair of stages read the same K block
+      const __nv_bfloat16* src[kRounds];
+      uint32_t active = 0;  // bit b: the lane has a row to fetch in round b
 #pragma unroll
       for (int b = 0; b < kRounds; ++b) {
-        if (((active >> b) & 1u) && x_off[b] >= 0) {
-          const uint32_t dst = st + dst_off[b & 1] + (b >> 1) * 1024u;
-          ptx::cp_async_16(dst, src + x_off[b], true);
-          if (second_half) ptx::cp_async_16(dst + kTokens * 128u, src + x_off[b] + 64, true);
-        }
+        const int32_t slot = static_cast<int32_t>(r0) + 4 * b;
+        const int32_t row = slot < t.ntok ? x_row_of(p, t, slot) : p.x_rows;
+        const bool has = row < p.x_rows;
+        src[b] = p.x + (has ? row * p.k : 0) + kb * kDecStageK + piece * 8;
+        active |= has ? 1u << b : 0u;
       }
-      ptx::cp_async_arrive_noinc(full);
-      cur.advance(stages);
+      const int32_t rounds = (t.ntok + 3) >> 2;
+      int32_t w_row = t.expert * (p.k / 16) + kb * (kDecStageK / 16);
+      int32_t s_row = t.expert * (p.k / 32) + kb * (kDecStageK / 32);
+      for (int32_t step = seg.kb; step < seg.ke; ++step) {
+        const int32_t w_col = t.n0 + (fuse ? (step & 1) * (p.n >> 1) : 0);
+        ptx::mbar_wait_sticky(empty0 + cur.s * 8u, cur.ph ^ 1u, abort_addr, bad);
+        bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
+        if (bad != 0) break;
+        const uint32_t st = ring0 + cur.s * kStageBytes;
+        const uint32_t full = full0 + cur.s * 8u;
+        if (lane == 0) {
+          ptx::mbar_arrive_expect_tx(full, kDecWSBytes);
+          ptx::tma_load_2d(st + kXBytes, &tm_w, full, 2 * w_col, w_row);
+          ptx::tma_load_2d(st + kXBytes + kDecWBytes, &tm_s, full, w_col, s_row);
+        }
+        __syncwarp();
+        const bool second_half = !(k_tail_half && step == k_steps - 1);
+#pragma unroll
+        for (int b = 0; b < kRounds; ++b) {
+          if (b >= rounds) break;
+          if ((active >> b) & 1u) {
+            const uint32_t dst = st + dst_off[b & 1] + (b >> 1) * 1024u;
+            ptx::cp_async_16(dst, src[b], true);
+            if (second_half) ptx::cp_async_16(dst + kTokens * 128u, src[b] + 64, true);
+          }
+        }
+        ptx::cp_async_arrive_noinc(full);
+        if (!kFuse || (step & 1)) {
+#pragma unroll
+          for (int b = 0; b < kRounds; ++b) src[b] += kDecStageK;
+          w_row += kDecStageK / 16;
+          s_row += kDecStageK / 32;
+        }
+        cur.advance(stages);
+      }
     }
     // Nothing may stay in flight towards shared memory when the CTA retires, also when the
     // computing warps give up after this warp has issued its last stage: the gathers and the
@@ -591,6 +568,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     __syncwarp();
   } else {
     // ---------------------------------------------------------- computing warps --
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const uint32_t q = (warp - kDecWorkers) & 3u;  // 32 weight rows of the tile
     const uint32_t wt = q * 32u + lane;            // 0..127 inside the worker
     const uint32_t bar_id = 1 + wk;
@@ -613,7 +591,8 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       } else if (kTokens == 16 || t.ntok <= 16) {
         decode_segment<kTokens, 2, 1 + fuse>(p, seg, t, ring, tail, q, lane, wt, bar_id, worker_id, stage);
       } else if constexpr (kTokens > 16) {
-        decode_segment<kTokens, 4, 1 + fuse>(p, seg, t, ring, tail, q, lane, wt, bar_id, worker_id, stage);
+        if (t.ntok <= 24) decode_segment<kTokens, 3, 1 + fuse>(p, seg, t, ring, tail, q, lane, wt, bar_id, worker_id, stage);
+        else decode_segment<kTokens, 4, 1 + fuse>(p, seg, t, ring, tail, q, lane, wt, bar_id, worker_id, stage);
       }
     }
     if (ring.bad != 0 && lane == 0 && p.status) atomicOr(p.status, kStatusDequantTimeout);
