@@ -100,9 +100,9 @@ inline cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 bloc
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
-// The same launch as clusters of two CTAs along x (grid.x even).
+// The same launch as clusters of `cluster` CTAs along x (grid.x a multiple of it).
 template <typename... Params, typename... Args>
-inline cudaError_t launch_kernel_pairs(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+inline cudaError_t launch_kernel_clusters(void (*kernel)(Params...), int cluster, dim3 grid, dim3 block, size_t smem,
                                        cudaStream_t stream, bool pdl, Args&&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
@@ -111,7 +111,7 @@ inline cudaError_t launch_kernel_pairs(void (*kernel)(Params...), dim3 grid, dim
   config.stream = stream;
   cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = 2;
+  attribute[0].val.clusterDim.x = static_cast<unsigned>(cluster);
   attribute[0].val.clusterDim.y = 1;
   attribute[0].val.clusterDim.z = 1;
   attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -67,13 +67,13 @@ silu_mul_routed_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __re
   }
 }
 
-template <int kWarps, int kBatch>
+template <int kWarps, int kBatch, int kCtas>
 __global__ void __launch_bounds__(kWarps * 32)
 moe_align_kernel(const int32_t* __restrict__ topk_ids, int32_t numel, int32_t expert_base,
                  int32_t num_experts, int32_t block_m, int32_t* __restrict__ sorted_ids,
                  int32_t sorted_cap, int32_t* __restrict__ expert_ids, int32_t expert_cap,
                  int32_t* __restrict__ num_tokens_padded) {
-  moe_align_block<kWarps, kBatch>(topk_ids, numel, numel, expert_base, num_experts, block_m, sorted_ids,
+  moe_align_block<kWarps, kBatch, kCtas>(topk_ids, numel, numel, expert_base, num_experts, block_m, sorted_ids,
                                   sorted_cap, expert_ids, expert_cap, num_tokens_padded);
 }
 
@@ -142,31 +142,41 @@ int chord_b200_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int6
                 static_cast<long long>(sorted_cap), static_cast<long long>(need / block_m * block_m));
   CHORD_REQUIRE(expert_cap >= need / block_m, "expert_ids capacity %lld is below the worst case %lld",
                 static_cast<long long>(expert_cap), static_cast<long long>(need / block_m));
-  // From 4096 ids on 32 warps, sixteen rounds of loads ahead, where the counters fit 160 KB (up
-  // to 1241 experts).  Below that the short loop of 16 warps: a batch's unrolled code costs a
-  // small call more (instruction fetches) than the loads it overlaps.
-  // (32768 ids over 48 experts: 39.6 us with a load per round and 16 warps, 18.5 us now; 2048 ids:
-  // 5.0 us with the short loop, 5.8 with the long one.)
-  constexpr size_t kMaxSmem = 160 * 1024;
+  // From 4096 ids on a cluster of eight CTAs of 32 warps (four rounds of loads ahead), where
+  // the counters fit 170 KB (up to 1279 experts).  Below that one CTA of 16 warps, with four rounds ahead
+  // from 513 ids on; up to 512 a warp has one round, and the batch's unrolled code would only
+  // cost instruction fetches.  (48 of 384 experts, us, one CTA with sixteen rounds ahead from 4096 ids on
+  // and one below / now: 32768 ids 19.6 / 6.9, 2048 ids 7.1 / 4.9.)
+  constexpr size_t kMaxSmem = 170 * 1024;
   const bool wide = numel >= 4096 && chord::moe_align_smem_bytes(num_experts, chord::kAlignWarps) <= kMaxSmem;
   const int warps = wide ? chord::kAlignWarps : chord::kAlignWarpsFew;
-  const auto kernel = wide ? chord::moe_align_kernel<chord::kAlignWarps, 16>
-                           : chord::moe_align_kernel<chord::kAlignWarpsFew, 1>;
+  const int which = wide ? 2 : (numel > 32 * chord::kAlignWarpsFew ? 1 : 0);
+  using Kernel = void (*)(const int32_t*, int32_t, int32_t, int32_t, int32_t, int32_t*, int32_t, int32_t*, int32_t, int32_t*);
+  static const Kernel kernels[3] = {chord::moe_align_kernel<chord::kAlignWarpsFew, 1, 1>,
+                                    chord::moe_align_kernel<chord::kAlignWarpsFew, 4, 1>,
+                                    chord::moe_align_kernel<chord::kAlignWarps, 4, chord::kAlignCtas>};
+  const Kernel kernel = kernels[which];
   const size_t smem = chord::moe_align_smem_bytes(num_experts, warps);
-  static bool attr_set[2][64] = {};
+  static bool attr_set[3][64] = {};
   int device = 0;
   CHORD_CUDA(cudaGetDevice(&device));
-  if (smem > 48 * 1024 && !attr_set[wide][device & 63]) {
+  if (smem > 48 * 1024 && !attr_set[which][device & 63]) {
     CHORD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    attr_set[wide][device & 63] = true;
+    attr_set[which][device & 63] = true;
   }
-  kernel<<<1, warps * 32, smem, static_cast<cudaStream_t>(stream)>>>(
-      topk_ids, static_cast<int32_t>(numel), static_cast<int32_t>(expert_base),
-      static_cast<int32_t>(num_experts), static_cast<int32_t>(block_m), sorted_ids,
-      static_cast<int32_t>(sorted_cap < (1ll << 30) ? sorted_cap : (1ll << 30)), expert_ids,
-      static_cast<int32_t>(expert_cap < (1ll << 30) ? expert_cap : (1ll << 30)),
-      num_tokens_padded);
-  CHORD_CUDA(cudaGetLastError());
+  const auto cap = [](int64_t v) { return static_cast<int32_t>(v < (1ll << 30) ? v : (1ll << 30)); };
+  const int32_t n = static_cast<int32_t>(numel), base = static_cast<int32_t>(expert_base);
+  const int32_t experts = static_cast<int32_t>(num_experts), block = static_cast<int32_t>(block_m);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (wide) {
+    CHORD_CUDA(chord::launch_kernel_clusters(kernel, chord::kAlignCtas, dim3(chord::kAlignCtas), dim3(warps * 32), smem, s,
+                                             false, topk_ids, n, base, experts, block, sorted_ids, cap(sorted_cap),
+                                             expert_ids, cap(expert_cap), num_tokens_padded));
+  } else {
+    kernel<<<1, warps * 32, smem, s>>>(topk_ids, n, base, experts, block, sorted_ids, cap(sorted_cap), expert_ids,
+                                       cap(expert_cap), num_tokens_padded);
+    CHORD_CUDA(cudaGetLastError());
+  }
   return chord::kOk;
 }
 

@@ -191,7 +191,7 @@ int launch_with_groups(const CUtensorMap& tm_w, const CUtensorMap& tm_s, const C
   const Kernel kernel = kernels[p.pair ? 2 : (hold ? 1 : 0)];
   if (p.pair) {
     // every CTA has to be resident (stream-K owners wait for their contributors)
-    CHORD_CUDA(launch_kernel_pairs(kernel, dim3(grid), dim3(threads), smem, stream, p.pdl != 0, tm_w, tm_s, tm_x, p));
+    CHORD_CUDA(launch_kernel_clusters(kernel, 2, dim3(grid), dim3(threads), smem, stream, p.pdl != 0, tm_w, tm_s, tm_x, p));
     return kOk;
   }
   CHORD_CUDA(launch_kernel(kernel, dim3(grid), dim3(threads), smem, stream, p.pdl != 0, tm_w, tm_s, tm_x, p));

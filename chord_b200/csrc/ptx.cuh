@@ -501,6 +501,13 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   return r;
 }
 
+// Word at a shared-memory address of any CTA of the cluster (address from map_to_cta).
+__device__ __forceinline__ int32_t ld_cluster(uint32_t cluster_addr) {
+  int32_t v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
+
 // Arrival on a barrier of either CTA of the cluster (address from map_to_cta).
 // Default semantics (as for a local arrival): a cluster-scope release was measured to
 // double the dequant warps' time per stage; what the barrier orders here is tensor memory

@@ -26,6 +26,24 @@ def test_alignment_shapes(device, numel, experts, total, base):
     assert torch.equal(e.cpu()[: count // 16], re)
 
 
+@pytest.mark.parametrize("numel", [512, 513, 2048, 2049, 32767, 32768, 32769, 100000])
+@pytest.mark.parametrize("experts,total,base,block_m", [(48, 384, 144, 128), (3, 3, 0, 8), (1, 400, 7, 16), (1279, 1280, 1, 8),
+                                                        (1280, 1280, 0, 8)])
+def test_alignment_batches_and_clusters(device, numel, experts, total, base, block_m):
+    """One round and one batch of ids per warp and one more; the last number of experts whose
+    counters let a cluster of CTAs align, and the next; experts of very uneven popularity."""
+    import chord_b200
+
+    g = torch.Generator().manual_seed(numel + experts)
+    topk = (torch.rand((numel, 1), generator=g) ** 3 * total).to(torch.int32)
+    s, e, p = chord_b200.moe_align_block_size(topk.to(device), block_m, experts, expert_base=base)
+    rs, re, rp = O.align_routing_blocks(topk, block_m, experts, base)
+    count = int(p.item())
+    assert count == int(rp)
+    assert torch.equal(s.cpu()[:count], rs)
+    assert torch.equal(e.cpu()[: count // block_m], re)
+
+
 def test_alignment_ids_outside_every_range(device):
     import chord_b200
 
