@@ -83,15 +83,26 @@ def routing_block_m(block_m, limit: int) -> int:
     return block_m
 
 
+_PREPARED_WEIGHT = None
+
+
 def prepared_weight(weight, device: torch.device, *, dtype_error=ValueError):
     """A :class:`PreparedWeight` whose tensors agree with its recorded ``n, k, E`` and
     live, contiguous, on ``device``.  Returns ``(packed, scale, E, n, k)``."""
-    from .packing import PreparedWeight
+    global _PREPARED_WEIGHT
+    if _PREPARED_WEIGHT is None:  # (packing imports this module)
+        from .packing import PreparedWeight as _PREPARED_WEIGHT
 
-    if not isinstance(weight, PreparedWeight):
+    if not isinstance(weight, _PREPARED_WEIGHT):
         raise TypeError("weight must be a PreparedWeight from pack_w4a16()")
     n, k, e = weight.n, weight.k, weight.num_experts
     packed, scale = weight.packed, weight.scale
+    # All conditions in one expression first (half the time of the statements below, which say
+    # what is wrong when it does not hold).
+    if (packed.dtype is torch.int32 and scale.dtype is torch.bfloat16 and packed.shape == (e, k // 16, n * 2)
+            and scale.shape == (e, k // 32, n) and packed.device == device and scale.device == device
+            and packed.is_contiguous() and scale.is_contiguous()):
+        return packed, scale, e, n, k
     if packed.dtype != torch.int32 or scale.dtype != torch.bfloat16:
         raise dtype_error(
             f"packed weight must be int32 and its scale bfloat16, got {packed.dtype} / {scale.dtype}")
@@ -119,6 +130,25 @@ def bf16_output(outputs, shape: tuple[int, int], device: torch.device, *, exact_
             f"outputs must be contiguous BF16 {shape} on {device}, got {tuple(outputs.shape)} "
             f"on {outputs.device}")
     return outputs
+
+
+def routing_tensors(sorted_ids, expert_ids, num_tokens_padded, device: torch.device) -> None:
+    """The three routing tensors of ``indexed``: contiguous int32 on ``device``, two vectors and one
+    element.  All conditions in one expression first, then one by one for the message."""
+    int32 = torch.int32
+    if (isinstance(sorted_ids, torch.Tensor) and isinstance(expert_ids, torch.Tensor)
+            and isinstance(num_tokens_padded, torch.Tensor)
+            and sorted_ids.dtype is int32 and expert_ids.dtype is int32 and num_tokens_padded.dtype is int32
+            and sorted_ids.ndim == 1 and expert_ids.ndim == 1 and num_tokens_padded.ndim <= 1
+            and num_tokens_padded.numel() == 1 and device.type == "cuda"
+            and sorted_ids.device == device and expert_ids.device == device and num_tokens_padded.device == device
+            and sorted_ids.is_contiguous() and expert_ids.is_contiguous() and num_tokens_padded.is_contiguous()):
+        return
+    tensor("sorted_ids", sorted_ids, dtype=torch.int32, ndim=1, device=device)
+    tensor("expert_ids", expert_ids, dtype=torch.int32, ndim=1, device=device)
+    tensor("num_tokens_padded", num_tokens_padded, dtype=torch.int32, device=device)
+    if num_tokens_padded.numel() != 1 or num_tokens_padded.ndim > 1:
+        raise ValueError("num_tokens_padded must be a scalar or a one-element tensor")
 
 
 def routing_contract(sorted_ids, expert_ids, num_tokens_padded, block_m: int, routed_limit: int,

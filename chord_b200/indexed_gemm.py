@@ -170,11 +170,7 @@ def w4a16_indexed(
     packed, scale, num_experts, shape_n, shape_k = _checks.prepared_weight(weight, device)
     if inputs.size(1) != shape_k:
         raise ValueError(f"inputs K={inputs.size(1)} does not match the weight's K={shape_k}")
-    _checks.tensor("sorted_ids", sorted_ids, dtype=torch.int32, ndim=1, device=device)
-    _checks.tensor("expert_ids", expert_ids, dtype=torch.int32, ndim=1, device=device)
-    _checks.tensor("num_tokens_padded", num_tokens_padded, dtype=torch.int32, device=device)
-    if num_tokens_padded.numel() != 1 or num_tokens_padded.ndim > 1:
-        raise ValueError("num_tokens_padded must be a scalar or a one-element tensor")
+    _checks.routing_tensors(sorted_ids, expert_ids, num_tokens_padded, device)
     _checks.integer("top_k", top_k, minimum=1)
     routed_m = inputs.size(0) * top_k
     block_m = (select_block_m(shape_n, shape_k, num_experts, routed_m) if block_m is None
