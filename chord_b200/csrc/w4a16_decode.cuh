@@ -22,16 +22,20 @@
 //   * a computing warp owns 32 of the tile's 128 weight rows over the whole K range: per
 //     K16 it loads two words per lane and the token fragments, dequantises and multiplies.
 //     The four warps share a stage but never wait for one another inside a tile;
-//   * a tile runs with 8, 16 or 32 token columns, by the rows it really has: at decode
+//   * a tile runs with 8, 16, 24 or 32 token columns, by the rows it really has: at decode
 //     sizes most routing blocks of 16 hold at most 8.
 //
-// Measured on a B200, gate_up [4096, 7168] / down [7168, 2048] of a layer's local experts, top-8
-// of 384, weights from HBM, replayed graph, tcgen05 version -> this one: 1 token (one expert
-// reached) 19.2 / 14.7 -> 12.8 / 10.3 us (no tensor memory to allocate, no activation buffer to
-// clear), 16 tokens (11 experts) 53.7 / 34.5 -> 44.0 / 27.8 us, 64 tokens (34) 134 / 80 -> 111 / 65 us,
-// 256 tokens (48) 188 / 111 -> 156 / 88 us (5.1 / 4.5 TB/s of packed weights and scales).
-// From 11 to 48 experts a launch takes 3.0 / 1.65 us per expert (5.5 / 5.0 TB/s) and 11 / 10 us
-// beside them: set-up, the first stages, and the stream-K slices at the end.
+// Measured on a B200, gate_up [4096, 7168] / down [7168, 2048] of a layer's local experts, weights
+// from HBM, replayed graph, us: tcgen05 version / with 15 instructions of dequantisation per word /
+// now: 1 expert reached 19.2, 14.7 / 13.2, 10.0 / 12.8, 9.8; 11 experts of 1 row 53.7, 34.5 / 44.8, 28.5 /
+// 42.1, 27.0; 48 of 5 rows 188, 111 / 153.5, 85.4 / 137.8, 78.0 (5.8 / 5.1 TB/s of packed weights and
+// scales).  These are bursts at 1965 MHz, where the latency of the warps' work bounds it; in steady
+// state the power cap does, and the last takes 157 / 83 us at about 1.7 GHz.  About 10 us per
+// launch do not depend on the experts: set-up, the first stages, and the stream-K slices at the end.
+//
+// Registers: 640 threads may have 96 each, which the wider tiles and fused gate_up spill; the four
+// feeder warps keep 56 and the computing warps take 104 (4 x 56 + 16 x 104 <= 20 x 96).  48 experts of
+// 14 rows (Poisson) 237 / 132 -> 227 / 125 us, with the 24-column tiles.
 #pragma once
 
 #include "w4a16_gemm.cuh"
