@@ -692,7 +692,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         const uint32_t mask = __ballot_sync(0xffffffffu, emit);
         carry_expert = __shfl_sync(0xffffffffu, e, 31);
         carry_start = __shfl_sync(0xffffffffu, run_start, 31);
-        __syncwarp();  // this round's blocks have been read
+        __syncwarp();  // all 32 blocks have been read
         if (emit) {
           const int32_t at = count + __popc(mask & ((1u << lane) - 1u));
           sh.tile_rows[at] = static_cast<uint16_t>(merged ? 128 + next_rows : rows);
