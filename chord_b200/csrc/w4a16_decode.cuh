@@ -120,6 +120,7 @@ __device__ __forceinline__ float silu_f32(float v) { return v / (1.0f + __expf(-
 struct DecodeLane {
   uint32_t w;      // packed words: slabs 2(q&1), 2(q&1)+1 of the 64-row chunk q>>1
   uint32_t s;      // scales of the same rows
+  uint32_t probe;  // those of K32 group lane % 4
   uint32_t x[4];   // ldmatrix row addresses for the K16 steps of a 64-wide K half
 };
 
@@ -159,89 +160,87 @@ __device__ __forceinline__ void decode_tokens(uint32_t addr, uint32_t (&b)[2 * N
   }
 }
 
-// decode_half() below for any scale: a loop over the two K32 groups, small code that is hardly
-// ever run.
+// What a lane reads of one 64-wide K half: 32 weight rows, and the tokens where there are 8.
+template <int NT>
+struct DecodeHalf {
+  uint2 words[4], scales[2];
+  uint32_t tokens[NT == 1 ? 8 : 1];  // fragments of the four K16 steps (loaded as they are needed for NT > 1)
+};
+
 template <int kTokens, int NT, int kHalf>
-__device__ __forceinline__ void decode_half_any(uint32_t st, const DecodeLane& at, float (&acc)[2][NT][4]) {
+__device__ __forceinline__ void decode_load(uint32_t st, const DecodeLane& at, DecodeHalf<NT>& h) {
   constexpr int kW = kTokens * 256 + 4096 * kHalf;
   constexpr int kS = kTokens * 256 + kDecWBytes + 512 * kHalf;
   constexpr int kX = kTokens * 128 * kHalf;
-#pragma unroll 1
-  for (uint32_t g = 0; g < 2; ++g) {
-    const uint2 scales = ptx::lds64<kS>(st + at.s + g * 256u);
-    uint2 words[2];
-    words[0] = ptx::lds64<kW>(st + at.w + g * 2048u);
-    words[1] = ptx::lds64<kW + 1024>(st + at.w + g * 2048u);
-    uint32_t b[2][2 * NT];
-    if constexpr (NT == 1) {
-      uint32_t t[4];
-      ptx::ldmatrix_x4<kX>(st + (at.x[0] ^ (g * 64u)), t);
-      b[0][0] = t[0];
-      b[0][1] = t[1];
-      b[1][0] = t[2];
-      b[1][1] = t[3];
-    } else {
-#pragma unroll
-      for (uint32_t j = 0; j < 2; ++j) decode_tokens<NT, kX>(st + (at.x[0] ^ (g * 64u + j * 32u)), b[j]);
-    }
+  h.words[0] = ptx::lds64<kW>(st + at.w);
+  h.words[1] = ptx::lds64<kW + 1024>(st + at.w);
+  h.words[2] = ptx::lds64<kW + 2048>(st + at.w);
+  h.words[3] = ptx::lds64<kW + 3072>(st + at.w);
+  h.scales[0] = ptx::lds64<kS>(st + at.s);
+  h.scales[1] = ptx::lds64<kS + 256>(st + at.s);
+  if constexpr (NT == 1) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      uint32_t a[4];
-      dequant_fragment_any(words[j].x, scales.x, a[0], a[1], a[2], a[3]);
+      uint32_t t[4];
+      ptx::ldmatrix_x4<kX>(st + at.x[j], t);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
-      dequant_fragment_any(words[j].y, scales.y, a[0], a[1], a[2], a[3]);
-#pragma unroll
-      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], a, b[j][2 * n], b[j][2 * n + 1]);
+      for (int i = 0; i < 4; ++i) h.tokens[4 * j + i] = t[i];
     }
   }
 }
 
-// One 64-wide K half of a stage: 32 weight rows x 64 K x 8 NT tokens.
-template <int kTokens, int NT, int kHalf>
-__device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, float (&acc)[2][NT][4]) {
-  constexpr int kW = kTokens * 256 + 4096 * kHalf;
-  constexpr int kS = kTokens * 256 + kDecWBytes + 512 * kHalf;
+// The products of one K half: 32 weight rows x 64 K x 8 NT tokens.
+template <int kTokens, int NT, int kHalf, bool kAnyScale>
+__device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, const DecodeHalf<NT>& h,
+                                            float (&acc)[2][NT][4]) {
   constexpr int kX = kTokens * 128 * kHalf;
-  uint2 words[4], scales[2];
-  words[0] = ptx::lds64<kW>(st + at.w);
-  words[1] = ptx::lds64<kW + 1024>(st + at.w);
-  words[2] = ptx::lds64<kW + 2048>(st + at.w);
-  words[3] = ptx::lds64<kW + 3072>(st + at.w);
-  scales[0] = ptx::lds64<kS>(st + at.s);
-  scales[1] = ptx::lds64<kS + 256>(st + at.s);
-  uint32_t b[4][2 * NT];  // token fragments of the four K16 steps
-  if constexpr (NT == 1) {
-    uint32_t t[4];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      ptx::ldmatrix_x4<kX>(st + at.x[j], t);
-      b[2 * j][0] = t[0];
-      b[2 * j][1] = t[1];
-      b[2 * j + 1][0] = t[2];
-      b[2 * j + 1][1] = t[3];
-    }
-  }
-  if (__any_sync(0xffffffffu, scales_out_of_range(scales[0], scales[1]) != 0)) {
-    decode_half_any<kTokens, NT, kHalf>(st, at, acc);
-    return;
-  }
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
-    const ScaleFactors fa = scale_factors(scales[g].x), fb = scale_factors(scales[g].y);
+    const Dequant<kAnyScale> da(h.scales[g].x), db(h.scales[g].y);
+    uint32_t a[2][4], c[2][4];
 #pragma unroll
-    for (int j = 2 * g; j < 2 * g + 2; ++j) {
-      if constexpr (NT > 1) decode_tokens<NT, kX>(st + at.x[j], b[j]);
-      uint32_t a[4], c[4];
-      dequant_fragment(words[j].x, fa, a[0], a[1], a[2], a[3]);
-      dequant_fragment(words[j].y, fb, c[0], c[1], c[2], c[3]);
+    for (int i = 0; i < 2; ++i) da(h.words[2 * g + i].x, a[i][0], a[i][1], a[i][2], a[i][3]);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a, b[j][2 * n], b[j][2 * n + 1]);
+    for (int i = 0; i < 2; ++i) db(h.words[2 * g + i].y, c[i][0], c[i][1], c[i][2], c[i][3]);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], c, b[j][2 * n], b[j][2 * n + 1]);
+    for (int i = 0; i < 2; ++i) {
+      const int j = 2 * g + i;
+      uint32_t b[2 * NT];
+      if constexpr (NT == 1) {
+        b[0] = h.tokens[2 * j];
+        b[1] = h.tokens[2 * j + 1];
+      } else {
+        decode_tokens<NT, kX>(st + at.x[j], b);
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[0][n], a[i], b[2 * n], b[2 * n + 1]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) ptx::mma_m16n8k16(acc[1][n], c[i], b[2 * n], b[2 * n + 1]);
     }
   }
+}
+
+// One stage whose first half has been loaded.
+template <int kTokens, int NT, bool kAnyScale>
+__device__ __forceinline__ void decode_stage_as(uint32_t st, const DecodeLane& at, bool second, DecodeHalf<NT>& h,
+                                                float (&acc)[2][NT][4]) {
+  decode_half<kTokens, NT, 0, kAnyScale>(st, at, h, acc);
+  if (second) {
+    decode_load<kTokens, NT, 1>(st, at, h);
+    decode_half<kTokens, NT, 1, kAnyScale>(st, at, h, acc);
+  }
+}
+
+// One stage.  Four lanes have the same scales, of its four K32 groups; each looks at the range of
+// one group's, and one vote settles both halves.
+template <int kTokens, int NT>
+__device__ __forceinline__ void decode_stage(uint32_t st, const DecodeLane& at, bool second, float (&acc)[2][NT][4]) {
+  DecodeHalf<NT> h;
+  const uint2 probe = ptx::lds64<kTokens * 256 + kDecWBytes>(st + at.probe);
+  decode_load<kTokens, NT, 0>(st, at, h);
+  if (small_scales(probe)) decode_stage_as<kTokens, NT, false>(st, at, second, h, acc);
+  else decode_stage_as<kTokens, NT, true>(st, at, second, h, acc);
 }
 
 // Ring position of a computing warp as running offsets (no multiplications in the loop).
@@ -267,6 +266,7 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
   DecodeLane at;
   at.w = (q >> 1) * 512u + lane * 16u + (q & 1) * 8u;
   at.s = (q >> 1) * 128u + (lane >> 2) * 16u + (q & 1) * 8u;
+  at.probe = at.s + (lane & 3u) * 256u;
   decode_x_offsets<NT>(lane, at.x);
   // Output row of token slot `lane`: loaded now, used in the epilogue.
   const int32_t rows = out_row_of(p, t, static_cast<int32_t>(lane));
@@ -289,15 +289,11 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
     for (int32_t kb = seg.kb; kb < seg.ke; ++kb) {
       const uint32_t st = ring.base + ring.off;
       ptx::mbar_wait_sticky<true>(ring.full0 + ring.bar, ring.ph, ring.abort_addr, ring.bad);
-      // (the last stage holds one K half only when K is an odd multiple of 64)
-      const bool second = !(tail && kb == seg.ke - 1);
-      if (kBlocks == 1 || (kb & 1) == 0) {
-        decode_half<kTokens, NT, 0>(st, at, acc[0]);
-        if (second) decode_half<kTokens, NT, 1>(st, at, acc[0]);
-      } else {
-        decode_half<kTokens, NT, 0>(st, at, acc[kBlocks - 1]);
-        if (second) decode_half<kTokens, NT, 1>(st, at, acc[kBlocks - 1]);
-      }
+      // (the last stage holds one K half only when K is an odd multiple of 64, which no fused call has:
+      // a branch less between its halves, 48 experts of 6 rows 150 -> 143 us)
+      const bool second = kBlocks == 2 || !(tail && kb == seg.ke - 1);
+      if (kBlocks == 1 || (kb & 1) == 0) decode_stage<kTokens, NT>(st, at, second, acc[0]);
+      else decode_stage<kTokens, NT>(st, at, second, acc[kBlocks - 1]);
       __syncwarp();
       ptx::mbar_arrive_lane0(ring.empty0 + ring.bar, lane);
       ring.off += kStageBytes;
@@ -379,8 +375,8 @@ __device__ __forceinline__ void decode_segment(const GemmParams& p, const Segmen
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float v = acc[0][m][n][i] * kWeightUnit;
-          if (kBlocks == 2) v = silu_f32(v) * (acc[kBlocks - 1][m][n][i] * kWeightUnit);
+          float v = acc[0][m][n][i];
+          if (kBlocks == 2) v = silu_f32(v) * acc[kBlocks - 1][m][n][i];
           stage[(2 * c + (i & 1)) * kDecPitch + 16 * m + 8 * (i >> 1) + g] = __float2bfloat16_rn(v);
         }
       __syncwarp();

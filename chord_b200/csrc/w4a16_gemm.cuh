@@ -62,11 +62,12 @@
 //
 // Numerics match the reference's kernels (humming/arith/mainloop_arith.cuh:66-101,
 // deep_gemm/ptx/ld_st.cuh:15-40): weight = RN_bf16((code - 8) * scale), products
-// and sums in FP32, one rounding to BF16 at the end.  (The operand and the sums carry a factor
-// 2^-6, see dequant_fragment.)
+// and sums in FP32, one rounding to BF16 at the end.
 #pragma once
 
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "ptx.cuh"
 #include "ring.h"
@@ -357,34 +358,37 @@ __device__ __forceinline__ int32_t out_row_of(const GemmParams& p, const TileInf
 // tcgen05.st.16x128b, which is also that of the A fragment of mma.m16n8k16:
 //   d0 = (row r,   K 2q..2q+1)     d1 = (row r+8, K 2q..2q+1)
 //   d2 = (row r,   K 2q+8..2q+9)   d3 = (row r+8, K 2q+8..2q+9)
-// each RN_bf16((code - 8) * scale) * 2^-6: the reference's weight times a power of two that the
-// epilogues take out again (kWeightUnit).  A factor 2^-6 in one operand scales every product and
-// every FP32 sum exactly, so that results are bit for bit those of unscaled weights.
+// each RN_bf16((code - 8) * scale), the reference's weight, subnormal ones included.
 //
 // One mask and one fused multiply-add per pair: a BF16 bit pattern below 0x100 is the number
 // pattern * 2^-133 (subnormals and the first binade have the same spacing), so a nibble in bits
 // 0-3 of a half is code * 2^-133 and one in bits 4-7 is code * 2^-129 as it stands; no exponent
-// has to be put in and its 128 taken out again.  Then code * 2^-133 * (scale * 2^127) - scale *
-// 2^-3 = (code - 8) * scale * 2^-6, rounded once, both factors exact in BF16.  Per word that
-// is one shift, four masks and four multiply-adds, and three multiplications per pair of
-// scales (shared by two words), where 128 + code, minus 136, times the scale takes three shifts,
-// four masks, four subtractions and four multiplications: the decode kernel, bound by the
-// instructions of its warps, went from 22 to 18 per word (48 experts of 4096 x 7168 / 7168 x
-// 2048, 5 rows each, us: 153.5 / 85.4 before, 142.3 / 80.1 now), the general one from 307 to 293 us
-// (48 of 4096 x 7168, 85 rows).  It needs |scale| < 2, so that scale * 2^127 stays finite; a warp that
-// meets another scale takes dequant_fragment_any for that K half.  (Weights below 2^-120 in
-// magnitude lose bits to the end of BF16's range.)
-constexpr float kWeightUnit = 64.0f;
+// has to be put in and its 128 taken out again.  Then code * 2^-133 * (scale * 2^133) - scale * 8 =
+// (code - 8) * scale, rounded once; both factors are exact in BF16 as long as scale * 2^133 stays
+// finite, which is |scale| < 2^-5 (weights of up to 1/4).  A warp that meets another scale in a
+// 128-wide stage takes dequant_fragment_any for that stage: 128 + code, minus 136, times the scale.
+//
+// Per word that is one shift, four masks and four multiply-adds, and two multiplications and two
+// additions per pair of scales (shared by two words), against three shifts, four masks, four
+// subtractions and four multiplications: the decode kernel is bound by the instructions of its
+// warps.  48 experts of 4096 x 7168, replayed graph in a burst, scales below 2^-5 / of 2^-5 and more, us: 5
+// rows each 136 / 160, 20 rows 213 / 239, 28 rows 261 / 279, 85 rows (general kernel) 286 / 315.
+constexpr uint32_t kSmallScaleEnd = 0x3D00u;  // 2^-5 as BF16
 
 struct ScaleFactors {
-  uint32_t lo, hi, off;  // scale * 2^127, scale * 2^123, scale * -2^-3; low half row r, high half row r+8
+  uint32_t lo, hi, off;  // scale * 2^133, scale * 2^129, scale * -8; low half row r, high half row r+8
 };
 
+// 2^127 is BF16's largest power of two, so the rest is added to the exponents: scale * 2^127 is a
+// normal number below 2^122 or zero.  (A zero becomes 2^-121, whose products with a code's 2^-129
+// vanish in the rounding.)
 __device__ __forceinline__ ScaleFactors scale_factors(uint32_t scales) {
   ScaleFactors f;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.lo) : "r"(scales), "r"(0x7F007F00u));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.hi) : "r"(scales), "r"(0x7D007D00u));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.off) : "r"(scales), "r"(0xBE00BE00u));
+  uint32_t t;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(scales), "r"(0x7F007F00u));
+  f.lo = t + 0x03000300u;
+  f.hi = t + 0x01000100u;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.off) : "r"(scales), "r"(0xC100C100u));
   return f;
 }
 
@@ -419,13 +423,7 @@ __device__ __forceinline__ void dequant_fragment(uint32_t w, const ScaleFactors&
       : "r"(w), "r"(f.lo), "r"(f.hi), "r"(f.off));
 }
 
-// Nonzero if one of the scales is 2 or more in magnitude, infinite or NaN.
-__device__ __forceinline__ uint32_t scales_out_of_range(uint2 a, uint2 b) {
-  return (a.x | a.y | b.x | b.y) & 0x40004000u;
-}
-
-// The same for any scale: 128 + code by way of the exponent, minus 136, times the scale, each
-// rounded, then times 2^-6 (exact).
+// For any scale, infinite and NaN ones too.
 __device__ __forceinline__ void dequant_fragment_any(uint32_t w, uint32_t scales, uint32_t& d0, uint32_t& d1,
                                                      uint32_t& d2, uint32_t& d3) {
   asm("{\n\t"
@@ -445,17 +443,36 @@ __device__ __forceinline__ void dequant_fragment_any(uint32_t w, uint32_t scales
       "sub.rn.bf16x2 v1, v1, %6;\n\t"
       "sub.rn.bf16x2 v2, v2, %6;\n\t"
       "sub.rn.bf16x2 v3, v3, %6;\n\t"
-      "mul.rn.bf16x2 v0, v0, lo;\n\t"
-      "mul.rn.bf16x2 v2, v2, hi;\n\t"
-      "mul.rn.bf16x2 v1, v1, lo;\n\t"
-      "mul.rn.bf16x2 v3, v3, hi;\n\t"
-      "mul.rn.bf16x2 %0, v0, %7;\n\t"
-      "mul.rn.bf16x2 %1, v2, %7;\n\t"
-      "mul.rn.bf16x2 %2, v1, %7;\n\t"
-      "mul.rn.bf16x2 %3, v3, %7;\n\t"
+      "mul.rn.bf16x2 %0, v0, lo;\n\t"
+      "mul.rn.bf16x2 %1, v2, hi;\n\t"
+      "mul.rn.bf16x2 %2, v1, lo;\n\t"
+      "mul.rn.bf16x2 %3, v3, hi;\n\t"
       "}\n"
       : "=&r"(d0), "=&r"(d1), "=&r"(d2), "=&r"(d3)
-      : "r"(w), "r"(scales), "r"(0x43084308u), "r"(0x3C803C80u));
+      : "r"(w), "r"(scales), "r"(0x43084308u));
+}
+
+
+// What two words with the same scales share, and one of them as a fragment.
+template <bool kAnyScale>
+struct Dequant {
+  ScaleFactors f;  // kAnyScale: f.lo is the scales
+  __device__ __forceinline__ explicit Dequant(uint32_t scales) {
+    if constexpr (kAnyScale) f.lo = scales;
+    else f = scale_factors(scales);
+  }
+  __device__ __forceinline__ void operator()(uint32_t w, uint32_t& d0, uint32_t& d1, uint32_t& d2, uint32_t& d3) const {
+    if constexpr (kAnyScale) dequant_fragment_any(w, f.lo, d0, d1, d2, d3);
+    else dequant_fragment(w, f, d0, d1, d2, d3);
+  }
+};
+
+// Whether all scales that the warp's lanes look at are below 2^-5 in magnitude; infinite and NaN
+// ones are not.  Must be called by all 32 lanes.
+__device__ __forceinline__ bool small_scales(uint2 scales) {
+  constexpr uint32_t carry = (0x8000u - kSmallScaleEnd) * 0x10001u;  // reaches the sign bit from the end on
+  const uint32_t over = (((scales.x & 0x7FFF7FFFu) + carry) | ((scales.y & 0x7FFF7FFFu) + carry)) & 0x80008000u;
+  return __all_sync(0xffffffffu, over == 0);
 }
 
 // Activation ring cut into sub-slots of 128 token rows (both 64-wide K halves, 32 KB).
@@ -1221,6 +1238,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // 64-row chunk q>>1) inside one K16 row of the stage, and of its four scales.
     const uint32_t w_off = (q >> 1) * 512u + lane * 16u + (q & 1) * 8u;
     const uint32_t s_off = (q >> 1) * 128u + (lane >> 2) * 16u + (q & 1) * 8u;
+    // Four lanes have the same scales, of the stage's four K32 groups; each looks at the range of one group's.
+    const uint32_t probe_off = s_off + (lane & 3u) * 256u;
     StageCursor cur, acur;
     uint32_t it = 0;
     // Two such warps per scheduler: bound by the latency of their own chain (wait, load,
@@ -1261,26 +1280,24 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         scales[g] = *reinterpret_cast<const uint2*>(ssrc + (2 * h + g) * 256);
       }
     };
-    auto dequant_half = [&](const uint2 (&words)[4], const uint2 (&scales)[2], uint32_t (&lo)[16],
-                            uint32_t (&hi)[16]) {
-      if (__any_sync(0xffffffffu, scales_out_of_range(scales[0], scales[1]) != 0)) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dequant_fragment_any(words[j].x, scales[j >> 1].x, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
-          dequant_fragment_any(words[j].y, scales[j >> 1].y, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
-        }
-        return;
-      }
+    // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
+    auto dequant_as = [&](auto any_scale, const uint2 (&words)[4], const uint2 (&scales)[2], uint32_t (&lo)[16],
+                          uint32_t (&hi)[16]) {
+      using Dq = Dequant<decltype(any_scale)::value>;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
-        // scales[g].x = {slab A row r, slab A row r+8}; .y = same for slab B.
-        const ScaleFactors fa = scale_factors(scales[g].x), fb = scale_factors(scales[g].y);
+        const Dq da(scales[g].x);
 #pragma unroll
-        for (int j = 2 * g; j < 2 * g + 2; ++j) {
-          dequant_fragment(words[j].x, fa, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
-          dequant_fragment(words[j].y, fb, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
-        }
+        for (int j = 2 * g; j < 2 * g + 2; ++j) da(words[j].x, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+        const Dq db(scales[g].y);
+#pragma unroll
+        for (int j = 2 * g; j < 2 * g + 2; ++j) db(words[j].y, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
       }
+    };
+    auto dequant_half = [&](const uint2 (&words)[4], const uint2 (&scales)[2], bool small, uint32_t (&lo)[16],
+                            uint32_t (&hi)[16]) {
+      if (small) dequant_as(std::false_type{}, words, scales, lo, hi);
+      else dequant_as(std::true_type{}, words, scales, lo, hi);
     };
     // Waits for the slot to be free, then stores one K half: lo to TMEM lanes 0-15 of
     // the quarter (first slab), hi to lanes 16-31 (second slab).
@@ -1320,7 +1337,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         uint2 words[4], scales[2];
         uint32_t lo[16], hi[16];
         load_half(wsrc, ssrc, 0, words, scales);
-        dequant_half(words, scales, lo, hi);
+        const uint2 probe = *reinterpret_cast<const uint2*>(smem_s + cur.s * kSStageBytes + probe_off);
+        const bool small = small_scales(probe);
+        dequant_half(words, scales, small, lo, hi);
         // Second half's words are fetched before the first half is stored, and the
         // stage goes back to the producers as soon as they are in registers.
         load_half(wsrc, ssrc, 1, words, scales);
@@ -1328,7 +1347,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         __syncwarp();
         ptx::mbar_arrive_lane0(wempty0 + cur.s * 8u, lane);
         store_half(a, aph, lo, hi);
-        dequant_half(words, scales, lo, hi);
+        dequant_half(words, scales, small, lo, hi);
         publish();  // this stage's first half
         store_half(a + 1, aph, lo, hi);
         bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
@@ -1448,8 +1467,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           ptx::tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const __nv_bfloat162 pair2 = __floats2bfloat162_rn(__uint_as_float(v[2 * j]) * kWeightUnit,
-                                                                __uint_as_float(v[2 * j + 1]) * kWeightUnit);
+            const __nv_bfloat162 pair2 = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
             held[i][j] = *reinterpret_cast<const uint32_t*>(&pair2);
           }
         }
@@ -1564,11 +1582,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             }
           }
         }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] *= kWeightUnit;
         if (fuse) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[j] = acc[j] / (1.0f + __expf(-acc[j])) * (up[j] * kWeightUnit);
+          for (int j = 0; j < 16; ++j) acc[j] = acc[j] / (1.0f + __expf(-acc[j])) * up[j];
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = __float2bfloat16_rn(acc[j]);
