@@ -300,19 +300,27 @@ int launch_decode(GemmParams p, const DeviceInfo& dev, const int32_t* packed, co
                                     w4a16_decode_kernel<32, false>};
   static std::once_flag flags[64];
   static cudaError_t attr_result[64];
+  static int short_of_registers[64];  // registers per thread of a kernel whose warps could not divide them
   int device = 0;
   CHORD_CUDA(cudaGetDevice(&device));
   std::call_once(flags[device & 63], [&] {
     for (const Kernel kernel : kernels) {
-      const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  dev.max_smem_optin);
+      cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            dev.max_smem_optin);
+      cudaFuncAttributes attributes = {};
+      if (rc == cudaSuccess) rc = cudaFuncGetAttributes(&attributes, kernel);
       if (attr_result[device & 63] == cudaSuccess) attr_result[device & 63] = rc;
+      if (rc == cudaSuccess && !decode_registers_fit(attributes.numRegs)) short_of_registers[device & 63] = attributes.numRegs;
     }
   });
   if (attr_result[device & 63] != cudaSuccess) {
-    return fail(kCudaError, "cudaFuncSetAttribute failed: %s",
+    return fail(kCudaError, "cudaFuncSetAttribute or cudaFuncGetAttributes failed: %s",
                 cudaGetErrorString(attr_result[device & 63]));
   }
+  // (the one wait in the kernel that has no limit of its own)
+  CHORD_REQUIRE(short_of_registers[device & 63] == 0,
+                "internal: the decode kernel was compiled to %d registers per thread, too few for its warps' shares",
+                short_of_registers[device & 63]);
   const Kernel kernel = kernels[p.mma_n > 16 ? 2 : (p.fuse_silu ? 1 : 0)];
   CHORD_CUDA(launch_kernel(kernel, dim3(grid), dim3(kDecThreads), smem, stream, p.pdl != 0, tm_w, tm_s, p));
   return kOk;

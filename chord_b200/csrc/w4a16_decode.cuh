@@ -38,6 +38,7 @@
 // 14 rows (Poisson) 237 / 132 -> 227 / 125 us, with the 24-column tiles.
 #pragma once
 
+#include "launch_rules.h"
 #include "w4a16_gemm.cuh"
 
 namespace chord {
@@ -50,6 +51,17 @@ constexpr int kDecMaxStages = 6;
 constexpr int kDecMaxTokens = 32;
 constexpr int kDecWorkers = 4;                        // workers per CTA
 constexpr int kDecThreads = 32 * (kDecWorkers + 4 * kDecWorkers);  // feeders, computing warps
+// Registers of a feeder's and of a computing warp's threads, once they have divided them
+// (setmaxnreg: multiples of 8, by whole warpgroups of four warps).
+constexpr int kDecFeederRegs = 56, kDecComputeRegs = 104;
+static_assert(kDecWorkers == 4 && kDecFeederRegs % 8 == 0 && kDecComputeRegs % 8 == 0, "setmaxnreg");
+
+// Whether the division is possible with what a kernel compiled to `num_regs` is launched with.
+constexpr bool decode_registers_fit(int num_regs) {
+  return register_split_fits(num_regs, kDecWorkers, kDecFeederRegs, 4 * kDecWorkers, kDecComputeRegs);
+}
+static_assert(decode_registers_fit(65536 / kDecThreads / 8 * 8), "the registers of an SM");
+
 constexpr int kDecPitch = 40;  // BF16 per token row of the epilogue buffer: 32 rows, padded against bank conflicts
 
 struct __align__(16) DecodeWorkerShared {
@@ -488,7 +500,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const uint32_t empty0 = ptx::smem_u32(&ws.empty[0]);
 
   if (warp < kDecWorkers) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDecFeederRegs));
     // ------------------------- feeder of worker `warp`: weights, scales, activations --
     // Lane 0 issues the two TMA boxes of a stage; all lanes gather its activation rows with
     // cp.async (lane l fetches the 16-byte piece l % 8 of rows l / 8 + 4 b, b < kTokens / 4,
@@ -568,7 +580,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     __syncwarp();
   } else {
     // ---------------------------------------------------------- computing warps --
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDecComputeRegs));  // (launch_decode has checked that they are there)
     const uint32_t q = (warp - kDecWorkers) & 3u;  // 32 weight rows of the tile
     const uint32_t wt = q * 32u + lane;            // 0..127 inside the worker
     const uint32_t bar_id = 1 + wk;
