@@ -3,6 +3,8 @@
 // sorted_ids / expert_ids / num_tokens_padded contract `indexed` consumes.
 #include <cuda_bf16.h>
 
+#include <mutex>
+
 #include "../../include/chord_b200.h"
 #include "common.h"
 #include "ptx.cuh"
@@ -77,6 +79,40 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, int32_t numel, int32_t ex
                                   sorted_cap, expert_ids, expert_cap, num_tokens_padded);
 }
 
+using AlignFn = void (*)(const int32_t*, int32_t, int32_t, int32_t, int32_t, int32_t*, int32_t, int32_t*, int32_t, int32_t*);
+const AlignFn kAlignKernels[3] = {moe_align_kernel<kAlignWarpsFew, 1, 1>, moe_align_kernel<kAlignWarpsFew, 4, 1>,
+                                  moe_align_kernel<kAlignWarps, 4, kAlignCtas>};
+
+// Whether the device can place the cluster at its largest, asked once per device.
+bool align_cluster_fits(int device) {
+  static std::mutex mutex;
+  static int answer[64];  // 0 = not asked yet, 1 = no, 2 = yes
+  std::lock_guard<std::mutex> guard(mutex);
+  int& known = answer[device & 63];
+  if (known == 0) {
+    const AlignFn kernel = kAlignKernels[static_cast<int>(AlignKernel::kCluster)];
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = kAlignCtas;
+    attribute[0].val.clusterDim.y = 1;
+    attribute[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(kAlignCtas);
+    config.blockDim = dim3(kAlignWarps * 32);
+    config.dynamicSmemBytes = kAlignMaxSmem;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlignMaxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    known = clusters >= 1 ? 2 : 1;
+  }
+  return known == 2;
+}
+
 }  // namespace
 }  // namespace chord
 
@@ -142,33 +178,24 @@ int chord_b200_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int6
                 static_cast<long long>(sorted_cap), static_cast<long long>(need / block_m * block_m));
   CHORD_REQUIRE(expert_cap >= need / block_m, "expert_ids capacity %lld is below the worst case %lld",
                 static_cast<long long>(expert_cap), static_cast<long long>(need / block_m));
-  // From 4096 ids on a cluster of eight CTAs of 32 warps (four rounds of loads ahead), where
-  // the counters fit 170 KB (up to 1279 experts).  Below that one CTA of 16 warps, with four rounds ahead
-  // from 513 ids on; up to 512 a warp has one round, and the batch's unrolled code would only
-  // cost instruction fetches.  (48 of 384 experts, us, one CTA with sixteen rounds ahead from 4096 ids on
-  // and one below / now: 32768 ids 19.6 / 6.9, 2048 ids 7.1 / 4.9.)
-  constexpr size_t kMaxSmem = 170 * 1024;
-  const bool wide = numel >= 4096 && chord::moe_align_smem_bytes(num_experts, chord::kAlignWarps) <= kMaxSmem;
-  const int warps = wide ? chord::kAlignWarps : chord::kAlignWarpsFew;
-  const int which = wide ? 2 : (numel > 32 * chord::kAlignWarpsFew ? 1 : 0);
-  using Kernel = void (*)(const int32_t*, int32_t, int32_t, int32_t, int32_t, int32_t*, int32_t, int32_t*, int32_t, int32_t*);
-  static const Kernel kernels[3] = {chord::moe_align_kernel<chord::kAlignWarpsFew, 1, 1>,
-                                    chord::moe_align_kernel<chord::kAlignWarpsFew, 4, 1>,
-                                    chord::moe_align_kernel<chord::kAlignWarps, 4, chord::kAlignCtas>};
-  const Kernel kernel = kernels[which];
-  const size_t smem = chord::moe_align_smem_bytes(num_experts, warps);
-  static bool attr_set[3][64] = {};
   int device = 0;
   CHORD_CUDA(cudaGetDevice(&device));
-  if (smem > 48 * 1024 && !attr_set[which][device & 63]) {
-    CHORD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    attr_set[which][device & 63] = true;
+  const bool cluster_fits = numel >= 4096 && chord::align_cluster_fits(device);
+  const chord::AlignKernel which = chord::align_kernel(numel, num_experts, cluster_fits);
+  const int warps = which == chord::AlignKernel::kCluster ? chord::kAlignWarps : chord::kAlignWarpsFew;
+  const chord::AlignFn kernel = chord::kAlignKernels[static_cast<int>(which)];
+  const size_t smem = chord::moe_align_smem_bytes(num_experts, warps);
+  static bool attr_set[3][64] = {};
+  bool& attr = attr_set[static_cast<int>(which)][device & 63];
+  if (smem > 48 * 1024 && !attr) {
+    CHORD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, chord::kAlignMaxSmem));
+    attr = true;
   }
   const auto cap = [](int64_t v) { return static_cast<int32_t>(v < (1ll << 30) ? v : (1ll << 30)); };
   const int32_t n = static_cast<int32_t>(numel), base = static_cast<int32_t>(expert_base);
   const int32_t experts = static_cast<int32_t>(num_experts), block = static_cast<int32_t>(block_m);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (wide) {
+  if (which == chord::AlignKernel::kCluster) {
     CHORD_CUDA(chord::launch_kernel_clusters(kernel, chord::kAlignCtas, dim3(chord::kAlignCtas), dim3(warps * 32), smem, s,
                                              false, topk_ids, n, base, experts, block, sorted_ids, cap(sorted_cap),
                                              expert_ids, cap(expert_cap), num_tokens_padded));

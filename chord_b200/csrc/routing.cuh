@@ -4,18 +4,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch_rules.h"
 #include "ptx.cuh"
 
 namespace chord {
-
-constexpr int kAlignWarps = 32;
-constexpr int kAlignWarpsFew = 16;
-constexpr int kAlignCtas = 8;  // of the cluster that aligns many ids
-
-// Dynamic shared memory the routine needs for `num_experts` experts.
-inline size_t moe_align_smem_bytes(int64_t num_experts, int warps) {
-  return ((static_cast<size_t>(warps) + 2) * num_experts + 1) * 4;
-}
 
 // kCtas CTAs (one, or a cluster) of kWarps warps each (CUDA form of the reference's
 // align_routing_blocks, tests/generators.py:192-230).  Pass 1 counts routes per (warp, expert);

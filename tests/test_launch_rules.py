@@ -37,3 +37,31 @@ def _run(tmp_path, source):
 
 def test_registers_of_the_decode_kernels_warps(tmp_path):
     assert _run(tmp_path, REGISTERS).returncode == 0
+
+
+ALIGNMENT = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "launch_rules.h"
+using namespace chord;
+
+int main() {
+  for (int64_t experts = 1; experts <= 2048; ++experts) {
+    for (int64_t numel : {0, 1, 512, 513, 4095, 4096, 32768, 1 << 30}) {
+      const bool counters_fit = moe_align_smem_bytes(experts, kAlignWarps) <= kAlignMaxSmem;
+      const AlignKernel with = align_kernel(numel, experts, true), without = align_kernel(numel, experts, false);
+      const AlignKernel one_cta = numel <= 512 ? AlignKernel::kShort : AlignKernel::kBatches;
+      // no cluster where the device cannot place one, and then the same CTA as elsewhere
+      if (without != one_cta) return std::printf("without a cluster: %lld ids, %lld experts\n", (long long)numel, (long long)experts), 1;
+      if (with != (numel >= 4096 && counters_fit ? AlignKernel::kCluster : one_cta)) return std::printf("with: %lld ids, %lld experts\n", (long long)numel, (long long)experts), 1;
+      if (moe_align_smem_bytes(experts, kAlignWarpsFew) > kAlignMaxSmem) return std::printf("%lld experts\n", (long long)experts), 1;
+    }
+  }
+  return 0;
+}
+"""
+
+
+def test_alignment_without_a_cluster(tmp_path):
+    done = _run(tmp_path, ALIGNMENT)
+    assert done.returncode == 0, done.stdout
