@@ -27,15 +27,16 @@
 //
 // Measured on a B200, gate_up [4096, 7168] / down [7168, 2048] of a layer's local experts, weights
 // from HBM, replayed graph, us: tcgen05 version / with 15 instructions of dequantisation per word /
-// now: 1 expert reached 19.2, 14.7 / 13.2, 10.0 / 12.8, 9.8; 11 experts of 1 row 53.7, 34.5 / 44.8, 28.5 /
-// 42.1, 27.0; 48 of 5 rows 188, 111 / 153.5, 85.4 / 137.8, 78.0 (5.8 / 5.1 TB/s of packed weights and
-// scales).  These are bursts at 1965 MHz, where the latency of the warps' work bounds it; in steady
-// state the power cap does, and the last takes 157 / 83 us at about 1.7 GHz.  About 10 us per
-// launch do not depend on the experts: set-up, the first stages, and the stream-K slices at the end.
+// now: 1 expert reached 19.2, 14.7 / 12.7, 10.2 / 12.2, 10.3; 11 experts of 1 row 53.7, 34.5 / 44.1, 27.4 /
+// 40.1, 25.9; 48 of 5 rows 188, 111 / 153.6, 85.5 / 137.3, 77.1 (5.8 / 5.2 TB/s of packed weights and
+// scales); 48 of 14 rows (Poisson) now 193, 110.  These are bursts at 1965 MHz, where the latency of the
+// warps' work bounds it; in steady state the power cap does: 48 of 5 rows 181, 96 / 168, 89 at 1.6 to 1.7
+// GHz.  About 10 us per launch do not depend on the experts: set-up, the first stages, and the
+// stream-K slices at the end.
 //
-// Registers: 640 threads may have 96 each, which the wider tiles and fused gate_up spill; the four
-// feeder warps keep 56 and the computing warps take 104 (4 x 56 + 16 x 104 <= 20 x 96).  48 experts of
-// 14 rows (Poisson) 237 / 132 -> 227 / 125 us, with the 24-column tiles.
+// Registers: 640 threads may have 96 each, of which the four feeder warps need 56 and the computing
+// warps, with wide tiles or two blocks of a fused gate_up, more than 96: those take 104 (4 x 56 + 16 x 104
+// <= 20 x 96), and only fused gate_up spills (8 bytes).
 #pragma once
 
 #include "launch_rules.h"

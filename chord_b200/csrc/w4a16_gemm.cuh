@@ -371,8 +371,10 @@ __device__ __forceinline__ int32_t out_row_of(const GemmParams& p, const TileInf
 // Per word that is one shift, four masks and four multiply-adds, and two multiplications and two
 // additions per pair of scales (shared by two words), against three shifts, four masks, four
 // subtractions and four multiplications: the decode kernel is bound by the instructions of its
-// warps.  48 experts of 4096 x 7168, replayed graph in a burst, scales below 2^-5 / of 2^-5 and more, us: 5
-// rows each 136 / 160, 20 rows 213 / 239, 28 rows 261 / 279, 85 rows (general kernel) 286 / 315.
+// warps.  48 experts of 4096 x 7168, replayed graph in a burst, us, a build with dequant_fragment_any
+// alone (without the later changes to the decode kernel) / scales of 2^-5 and more now / scales below
+// 2^-5 now: 5 rows each 154 / 158 / 138, 20 rows 276 / 234 / 214, 28 rows 279 / 274 / 261, 85 rows (general
+// kernel) 309 / 318 / 299.
 constexpr uint32_t kSmallScaleEnd = 0x3D00u;  // 2^-5 as BF16
 
 struct ScaleFactors {
@@ -1533,10 +1535,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           }
         }
         if constexpr (kPair) {
-          // On pairs the partial sums lie as [four columns][weight row][column]: 16-byte vectors, a
-          // warp's consecutive, two contributors' in flight (tiles have 256 columns, and the owner
-          // reads every contributor's).  24 groups of 4096 x 7168 and 7168 x 2048, 128 rows, whole
-          // layer, us: 378.8 with words, 377.1 with vectors; on single CTAs vectors cost 1 %.
+          // On pairs (mma_n a multiple of 16 above 128) the partial sums lie as [four columns][weight
+          // row][column]: 16-byte vectors, a warp's consecutive, two contributors' in flight.  Masked
+          // launches of 4096 x 7168 / 7168 x 2048, words -> vectors, us, three runs of each in turn within
+          // 0.4 of each other: 24 groups of 128 rows 191.6 -> 189.3 / 104.2 -> 103.7, 12 of 250 rows 138.7 ->
+          // 136.9 / 81.6 -> 79.2, 7 of 250 rows 87.1 -> 85.0 / 57.3 -> 55.3, 48 of 200 rows the same; on single
+          // CTAs vectors cost 1 %.
           if (seg.type != kSegFull) {
             float4* part = reinterpret_cast<float4*>(p.workspace + blockIdx.x * ws_slot + static_cast<size_t>(c0) * kBlockN) + et;
             if (seg.type == kSegContrib) {
