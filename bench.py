@@ -86,13 +86,17 @@ def measured_peaks():
 def recorded_traffic():
     """DRAM bytes per step of the decode kernel's two launches from the committed ncu
     capture (profiles/w4a16_decode_kernel_traffic.json), or None if there is none of the
-    kernel as it stands (the record holds the hash of the source it was captured on)."""
+    kernel as it stands (the record names the files the kernel was compiled from when it was
+    captured and holds the hash of their contents, one after the other)."""
     path = ROOT / "profiles" / "w4a16_decode_kernel_traffic.json"
     if not path.exists():
         return None
     record = json.loads(path.read_text())
-    source = ROOT / record["source"]
-    if not source.exists() or hashlib.sha256(source.read_bytes()).hexdigest() != record["source_sha256"]:
+    names = [record["source"]] if isinstance(record["source"], str) else record["source"]
+    sources = [ROOT / name for name in names]
+    if not all(source.exists() for source in sources):
+        return None
+    if hashlib.sha256(b"".join(source.read_bytes() for source in sources)).hexdigest() != record["source_sha256"]:
         return None
     return record
 
