@@ -210,7 +210,7 @@ __device__ __forceinline__ void decode_half(uint32_t st, const DecodeLane& at, c
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
-    const Dequant<kAnyScale> da(h.scales[g].x), db(h.scales[g].y);
+    const Dequant<kAnyScale, true> da(h.scales[g].x), db(h.scales[g].y);
     uint32_t a[2][4], c[2][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i) da(h.words[2 * g + i].x, a[i][0], a[i][1], a[i][2], a[i][3]);

@@ -368,28 +368,36 @@ __device__ __forceinline__ int32_t out_row_of(const GemmParams& p, const TileInf
 // finite, which is |scale| < 2^-5 (weights of up to 1/4).  A warp that meets another scale in a
 // 128-wide stage takes dequant_fragment_any for that stage: 128 + code, minus 136, times the scale.
 //
-// Per word that is one shift, four masks and four multiply-adds, and two multiplications and two
-// additions per pair of scales (shared by two words), against three shifts, four masks, four
+// Per word that is one shift, four masks and four multiply-adds, and four operations per pair of
+// scales (shared by two words), against three shifts, four masks, four
 // subtractions and four multiplications: the decode kernel is bound by the instructions of its
 // warps.  48 experts of 4096 x 7168, replayed graph in a burst, us, a build with dequant_fragment_any
-// alone (without the later changes to the decode kernel) / scales of 2^-5 and more now / scales below
-// 2^-5 now: 5 rows each 154 / 158 / 138, 20 rows 276 / 234 / 214, 28 rows 279 / 274 / 261, 85 rows (general
-// kernel) 309 / 318 / 299.
+// alone (without the later changes to both kernels) / scales of 2^-5 and more now / scales below
+// 2^-5 now: 5 rows each 155 / 158 / 137, 20 rows 276 / 235 / 215, 28 rows 280 / 276 / 261; general kernel, 60 rows
+// 279 / 292 / 256, 85 rows 305 / 317 / 290.
 constexpr uint32_t kSmallScaleEnd = 0x3D00u;  // 2^-5 as BF16
 
 struct ScaleFactors {
   uint32_t lo, hi, off;  // scale * 2^133, scale * 2^129, scale * -8; low half row r, high half row r+8
 };
 
-// 2^127 is BF16's largest power of two, so the rest is added to the exponents: scale * 2^127 is a
-// normal number below 2^122 or zero.  (A zero becomes 2^-121, whose products with a code's 2^-129
-// vanish in the rounding.)
+// 2^127 is BF16's largest power of two; the rest is multiplied too, or added to the exponents (scale *
+// 2^127 is a normal number below 2^122, or zero, which becomes 2^-121, whose products with a code's
+// 2^-129 vanish in the rounding).  The decode kernel adds, the general one multiplies: 48 experts of
+// 4096 x 7168, us, multiplying / adding: 5 rows 140 / 138, 20 rows 217 / 214, 28 rows 258 / 261 there, 40 rows 256 /
+// 260, fused 85 rows 316 / 319 here.
+template <bool kAddExponents>
 __device__ __forceinline__ ScaleFactors scale_factors(uint32_t scales) {
   ScaleFactors f;
   uint32_t t;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(scales), "r"(0x7F007F00u));
-  f.lo = t + 0x03000300u;
-  f.hi = t + 0x01000100u;
+  if constexpr (kAddExponents) {
+    f.lo = t + 0x03000300u;
+    f.hi = t + 0x01000100u;
+  } else {
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.lo) : "r"(t), "r"(0x42804280u));
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.hi) : "r"(t), "r"(0x40804080u));
+  }
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(f.off) : "r"(scales), "r"(0xC100C100u));
   return f;
 }
@@ -456,12 +464,12 @@ __device__ __forceinline__ void dequant_fragment_any(uint32_t w, uint32_t scales
 
 
 // What two words with the same scales share, and one of them as a fragment.
-template <bool kAnyScale>
+template <bool kAnyScale, bool kAddExponents>
 struct Dequant {
   ScaleFactors f;  // kAnyScale: f.lo is the scales
   __device__ __forceinline__ explicit Dequant(uint32_t scales) {
     if constexpr (kAnyScale) f.lo = scales;
-    else f = scale_factors(scales);
+    else f = scale_factors<kAddExponents>(scales);
   }
   __device__ __forceinline__ void operator()(uint32_t w, uint32_t& d0, uint32_t& d1, uint32_t& d2, uint32_t& d3) const {
     if constexpr (kAnyScale) dequant_fragment_any(w, f.lo, d0, d1, d2, d3);
@@ -1240,6 +1248,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // 64-row chunk q>>1) inside one K16 row of the stage, and of its four scales.
     const uint32_t w_off = (q >> 1) * 512u + lane * 16u + (q & 1) * 8u;
     const uint32_t s_off = (q >> 1) * 128u + (lane >> 2) * 16u + (q & 1) * 8u;
+    // Which scales a loop over stages takes: those below 2^-5, others, or both by a branch.
+    constexpr int kSmallOnly = 0, kAnyOnly = 1, kEither = 2;
     // Four lanes have the same scales, of the stage's four K32 groups; each looks at the range of one group's.
     const uint32_t probe_off = s_off + (lane & 3u) * 256u;
     StageCursor cur, acur;
@@ -1283,9 +1293,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       }
     };
     // scales[g].x = {slab A row r, slab A row r+8} of K32 group g; .y = the same for slab B.
-    auto dequant_as = [&](auto any_scale, const uint2 (&words)[4], const uint2 (&scales)[2], uint32_t (&lo)[16],
-                          uint32_t (&hi)[16]) {
-      using Dq = Dequant<decltype(any_scale)::value>;
+    auto dequant_half = [&](auto any_scale, const uint2 (&words)[4], const uint2 (&scales)[2], uint32_t (&lo)[16],
+                            uint32_t (&hi)[16]) {
+      using Dq = Dequant<decltype(any_scale)::value, false>;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         const Dq da(scales[g].x);
@@ -1296,10 +1306,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         for (int j = 2 * g; j < 2 * g + 2; ++j) db(words[j].y, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
       }
     };
-    auto dequant_half = [&](const uint2 (&words)[4], const uint2 (&scales)[2], bool small, uint32_t (&lo)[16],
-                            uint32_t (&hi)[16]) {
-      if (small) dequant_as(std::false_type{}, words, scales, lo, hi);
-      else dequant_as(std::true_type{}, words, scales, lo, hi);
+    auto dequant_half_as = [&](auto way, bool small, const uint2 (&words)[4], const uint2 (&scales)[2], uint32_t (&lo)[16],
+                               uint32_t (&hi)[16]) {
+      constexpr int kWay = decltype(way)::value;
+      if constexpr (kWay != kEither) dequant_half(std::bool_constant<kWay == kAnyOnly>{}, words, scales, lo, hi);
+      else if (small) dequant_half(std::false_type{}, words, scales, lo, hi);
+      else dequant_half(std::true_type{}, words, scales, lo, hi);
     };
     // Waits for the slot to be free, then stores one K half: lo to TMEM lanes 0-15 of
     // the quarter (first slab), hi to lanes 16-31 (second slab).
@@ -1329,31 +1341,50 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       it += first;
       cur.advance_by(first, w_stages);
       acur.advance_by(first, a_stages);
-      for (; it < it_end; it += kDequantGroups, cur.advance_by(kDequantGroups, w_stages),
-                          acur.advance_by(kDequantGroups, a_stages)) {
-        const uint32_t a = acur.s << 1;  // half-slots a (first K half) and a + 1 (second)
-        const uint32_t aph = acur.ph;
-        ptx::mbar_wait_sticky(wfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
-        const uint8_t* wsrc = smem_w + cur.s * kWStageBytes + w_off;
-        const uint8_t* ssrc = smem_s + cur.s * kSStageBytes + s_off;
-        uint2 words[4], scales[2];
-        uint32_t lo[16], hi[16];
-        load_half(wsrc, ssrc, 0, words, scales);
-        const uint2 probe = *reinterpret_cast<const uint2*>(smem_s + cur.s * kSStageBytes + probe_off);
-        const bool small = small_scales(probe);
-        dequant_half(words, scales, small, lo, hi);
-        // Second half's words are fetched before the first half is stored, and the
-        // stage goes back to the producers as soon as they are in registers.
-        load_half(wsrc, ssrc, 1, words, scales);
-        publish();  // previous stage's second half
-        __syncwarp();
-        ptx::mbar_arrive_lane0(wempty0 + cur.s * 8u, lane);
-        store_half(a, aph, lo, hi);
-        dequant_half(words, scales, small, lo, hi);
-        publish();  // this stage's first half
-        store_half(a + 1, aph, lo, hi);
-        bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
-        if (bad != 0) break;
+      // On single CTAs one loop per way to dequantise, each left at a stage that needs the other (which
+      // waits for and loads that stage again): with a branch in one loop a half jumps to code beside the loop
+      // and back, 48 experts of 60 rows, 4096 x 7168 / 7168 x 2048, us: 265 / 149, with two loops 256 / 138.  On
+      // pairs, which the products bound, the branch is the better (24 of 250 rows 279 / 146.5, 280.4 / 148.5).
+      auto run_stages = [&](auto way) {
+        constexpr int kWay = decltype(way)::value;
+        for (; it < it_end; it += kDequantGroups, cur.advance_by(kDequantGroups, w_stages),
+                            acur.advance_by(kDequantGroups, a_stages)) {
+          const uint32_t a = acur.s << 1;  // half-slots a (first K half) and a + 1 (second)
+          const uint32_t aph = acur.ph;
+          ptx::mbar_wait_sticky(wfull0 + cur.s * 8u, cur.ph, abort_addr, bad);
+          const uint8_t* wsrc = smem_w + cur.s * kWStageBytes + w_off;
+          const uint8_t* ssrc = smem_s + cur.s * kSStageBytes + s_off;
+          uint2 words[4], scales[2];
+          uint32_t lo[16], hi[16];
+          load_half(wsrc, ssrc, 0, words, scales);
+          const uint2 probe = *reinterpret_cast<const uint2*>(smem_s + cur.s * kSStageBytes + probe_off);
+          const bool small = small_scales(probe);
+          if (kWay != kEither && small == (kWay == kAnyOnly)) {
+            bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
+            return;
+          }
+          dequant_half_as(way, small, words, scales, lo, hi);
+          // Second half's words are fetched before the first half is stored, and the
+          // stage goes back to the producers as soon as they are in registers.
+          load_half(wsrc, ssrc, 1, words, scales);
+          publish();  // previous stage's second half
+          __syncwarp();
+          ptx::mbar_arrive_lane0(wempty0 + cur.s * 8u, lane);
+          store_half(a, aph, lo, hi);
+          dequant_half_as(way, small, words, scales, lo, hi);
+          publish();  // this stage's first half
+          store_half(a + 1, aph, lo, hi);
+          bad = __any_sync(0xffffffffu, bad != 0) ? 1u : 0u;
+          if (bad != 0) return;
+        }
+      };
+      while (bad == 0 && it < it_end) {
+        if constexpr (kPair) {
+          run_stages(std::integral_constant<int, kEither>{});
+        } else {
+          run_stages(std::integral_constant<int, kSmallOnly>{});
+          if (bad == 0 && it < it_end) run_stages(std::integral_constant<int, kAnyOnly>{});
+        }
       }
       // `it` overshoots the segment's end by less than one stride: bring the cursor back.
       if (bad == 0) {
