@@ -1,23 +1,10 @@
-// Rules of launches that hosts without a GPU can check too: plain C++.
+// Which kernel aligns a routing (routing.cuh): plain C++, so that a host without a GPU can check it too.
 #pragma once
 
 #include <cstddef>
 #include <cstdint>
 
 namespace chord {
-
-// Registers a thread has when a kernel is compiled to `num_regs` (the hardware hands them out in
-// eights).
-constexpr int allocated_registers(int num_regs) { return (num_regs + 7) / 8 * 8; }
-
-// Whether warps can divide their registers anew (setmaxnreg): what a CTA's warps take afterwards has to
-// come out of what it was launched with.  Otherwise the warps that ask for more wait for ever.
-constexpr bool register_split_fits(int num_regs, int less_warps, int less_regs, int more_warps, int more_regs) {
-  return less_warps * less_regs + more_warps * more_regs <= (less_warps + more_warps) * allocated_registers(num_regs) &&
-         less_regs <= allocated_registers(num_regs) && more_regs >= allocated_registers(num_regs);
-}
-
-// ---- routing alignment (routing.cuh)
 
 constexpr int kAlignWarps = 32;
 constexpr int kAlignWarpsFew = 16;
@@ -34,15 +21,16 @@ enum class AlignKernel { kShort = 0, kBatches = 1, kCluster = 2 };
 // From 4096 ids on a cluster of eight CTAs of 32 warps (four rounds of loads ahead), where
 // the counters fit 170 KB (up to 1279 experts) and the device can place such a cluster
 // (`cluster_fits`: a part of a GPU may have too few SMs side by side).  Otherwise one CTA of 16 warps, with
-// four rounds ahead from 513 ids on; up to 512 a warp has one round, and the batch's unrolled
-// code would only cost instruction fetches.
+// four rounds ahead from 513 ids on (more than the experts, where those are more); up to 512 a warp has
+// one round, and the batch's unrolled code would only cost instruction fetches.
 // One CTA / the cluster, us (replayed graph): 48 of 384 experts, 2048 ids 4.0 / 5.7, 4096 ids 5.7 / 5.8,
 // 6144 ids 7.0 / 5.7, 32768 ids 24.7 / 6.7; 384 experts, 2048 ids 7.0 / 8.7, 4096 ids 10.0 / 8.6.
-// One round / four rounds ahead: 48 of 384 experts, 1024 ids 4.2 / 3.6, 2048 ids 5.4 / 4.0; 1024 experts,
-// 1024 ids 8.4 / 8.8, 2048 ids 11.0 / 10.5.
+// One round / four rounds ahead: 48 of 384 experts, 1024 ids 4.2 / 3.6, 2048 ids 5.4 / 4.0; 640 experts, 640
+// ids 6.8 / 6.8, 1024 ids 7.4 / 7.4, 1280 ids 8.4 / 7.7; 1024 experts, 1024 ids 8.7 / 9.0, 1280 ids 9.7 / 9.3; 2048
+// experts, 1024 ids 12.5 / 13.7, 2048 ids 15.2 / 15.5.
 constexpr AlignKernel align_kernel(int64_t numel, int64_t num_experts, bool cluster_fits) {
   if (numel >= 4096 && cluster_fits && moe_align_smem_bytes(num_experts, kAlignWarps) <= kAlignMaxSmem) return AlignKernel::kCluster;
-  return numel > 32 * kAlignWarpsFew ? AlignKernel::kBatches : AlignKernel::kShort;
+  return numel > 32 * kAlignWarpsFew && numel > num_experts ? AlignKernel::kBatches : AlignKernel::kShort;
 }
 
 }  // namespace chord

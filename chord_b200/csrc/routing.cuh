@@ -4,7 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "launch_rules.h"
+#include "align_rules.h"
 #include "ptx.cuh"
 
 namespace chord {
@@ -74,7 +74,7 @@ __device__ __forceinline__ void moe_align_block(const int32_t* topk_ids, int32_t
       counts[w * num_experts + x] = run;
       run += c;
     }
-    totals[x] = run;
+    if constexpr (kCtas > 1) totals[x] = run;
     offsets[x] = (run + block_m - 1) / block_m * block_m;
   }
   if constexpr (kCtas > 1) {

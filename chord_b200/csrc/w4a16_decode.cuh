@@ -39,7 +39,7 @@
 // <= 20 x 96), and only fused gate_up spills (8 bytes).
 #pragma once
 
-#include "launch_rules.h"
+#include "register_split.h"
 #include "w4a16_gemm.cuh"
 
 namespace chord {

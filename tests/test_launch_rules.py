@@ -1,4 +1,4 @@
-"""The rules of launches in csrc/launch_rules.h, compiled for the host."""
+"""The rules of launches in csrc/register_split.h and csrc/align_rules.h, compiled for the host."""
 
 import shutil
 import subprocess
@@ -9,7 +9,7 @@ import pytest
 CSRC = Path(__file__).resolve().parents[1] / "chord_b200" / "csrc"
 
 REGISTERS = r"""
-#include "launch_rules.h"
+#include "register_split.h"
 using chord::register_split_fits;
 
 // Four warps go down to 56 registers, sixteen up to 104: 1888 of the 20 * 96 there are.
@@ -42,15 +42,15 @@ def test_registers_of_the_decode_kernels_warps(tmp_path):
 ALIGNMENT = r"""
 #include <cstdio>
 #include <initializer_list>
-#include "launch_rules.h"
+#include "align_rules.h"
 using namespace chord;
 
 int main() {
   for (int64_t experts = 1; experts <= 2048; ++experts) {
-    for (int64_t numel : {0, 1, 512, 513, 4095, 4096, 32768, 1 << 30}) {
+    for (int64_t numel : {0, 1, 512, 513, 1024, 1025, 2048, 2049, 4095, 4096, 32768, 1 << 30}) {
       const bool counters_fit = moe_align_smem_bytes(experts, kAlignWarps) <= kAlignMaxSmem;
       const AlignKernel with = align_kernel(numel, experts, true), without = align_kernel(numel, experts, false);
-      const AlignKernel one_cta = numel <= 512 ? AlignKernel::kShort : AlignKernel::kBatches;
+      const AlignKernel one_cta = numel <= 512 || numel <= experts ? AlignKernel::kShort : AlignKernel::kBatches;
       // no cluster where the device cannot place one, and then the same CTA as elsewhere
       if (without != one_cta) return std::printf("without a cluster: %lld ids, %lld experts\n", (long long)numel, (long long)experts), 1;
       if (with != (numel >= 4096 && counters_fit ? AlignKernel::kCluster : one_cta)) return std::printf("with: %lld ids, %lld experts\n", (long long)numel, (long long)experts), 1;
